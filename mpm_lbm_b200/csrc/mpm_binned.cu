@@ -1,17 +1,18 @@
-// Binned MPM substeps: particles sorted by 4x4x4-cell block and cut into
+// Binned MPM substeps: particles sorted by 8x8x8-cell block and cut into
 // chunks; one launch per substep, in which each CTA takes whole chunks
 // through the G2P gather of the previous substep (grid update evaluated while
 // the chunk's node box is staged), the P2G stress / reaction payload and the
-// P2G scatter staged in a shared-memory tile, flushed with one global atomic
-// per touched node value.  Three grid buffers rotate so that only the boxes
-// touched two substeps earlier are zeroed, by the launch after their last
-// reader.
+// P2G scatter, summed per chunk in shared memory and added to the grid with
+// one global atomic per touched node value.  Three grid buffers rotate so that
+// only the boxes touched two substeps earlier are zeroed, by the launch after
+// their last reader.
 //
 // The per-particle and per-node arithmetic is the one of the one-phase
 // kernels (mpm_common.cuh): solid.py:212-315 and the reaction transfers of
-// penalty.py:90-129, moving_boundary.py:58-110, link_area.py:84-193.  Only
-// the summation order of the grid sums differs (shared-memory atomics, then
-// one global atomic per chunk and touched node value).
+// penalty.py:90-129, moving_boundary.py:58-110, link_area.py:84-193.  The
+// order of the sums differs (stencils axis by axis, per-warp tiles, then one
+// global atomic per chunk and touched node value), and a node's velocity is
+// its momentum plus dt times its force, times one reciprocal of its mass.
 
 #include <cuda_runtime.h>
 
@@ -257,14 +258,14 @@ struct Box {
 
 __device__ __forceinline__ Box load_box(const int32_t* r) {
   Box b;
-  long long v = 1;
+  unsigned v = 1;  // extents of at most 1600 nodes (see layout()): below 2^32
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
     b.lo[a] = r[a];
     b.ext[a] = max(r[3 + a] - r[a] + 1, 0);
-    v *= b.ext[a];
+    v *= (unsigned)b.ext[a];
   }
-  b.vol = v > INT_MAX ? INT_MAX : (int)v;
+  b.vol = (int)min(v, (unsigned)INT_MAX);
   return b;
 }
 
@@ -274,46 +275,63 @@ __device__ __forceinline__ float bspline_w(float f, int o) {
   return o == 0 ? 0.5f * (1.5f - f) * (1.5f - f) : (o == 1 ? 0.75f - (f - 1.0f) * (f - 1.0f) : 0.5f * (f - 0.5f) * (f - 0.5f));
 }
 
-// Fallbacks for chunks whose node box does not fit the shared-memory tile
-// (bins gone stale): rolled loops, so that the staged path stays compact.
-__device__ __forceinline__ void g2p_gather_global(const FsiGrid& g, const FsiMpmParams& mp, const BSpline& b,
-                                                  float nvl[3], float nC[9]) {
+// One velocity component of a grid node of mass 1 / im after the grid update
+// and the sticky walls (solid.py:97-111, 251-259): momentum and dt times the
+// external force over the mass
+__device__ __forceinline__ float grid_node_component(float P, float im, float f, float gravity, int idx, int G,
+                                                     const FsiMpmParams& mp) {
+  float u = (P + mp.dt * f) * im + mp.dt * gravity;
+  if (idx < mp.bound && u < 0.0f) u = 0.0f;
+  if (idx > G - mp.bound && u > 0.0f) u = 0.0f;
+  return u;
+}
+
+// G2P sums of a particle whose stencil leaves the grid, or whose chunk's node
+// box does not fit the shared-memory stage (bins gone stale): a rolled loop
+// over the nodes inside the grid, from the stage when stg is non-null, from
+// the grid otherwise.
+__device__ __noinline__ void g2p_slow(const float* stg, int nv, const Box& bx, const FsiGrid& g, const FsiMpmParams& mp,
+                                      const BSpline& b, float s4, float v[3], float nC[9]) {
   const int G = g.n;
   const int64_t N = (int64_t)G * G * G;
-  const float s4 = 4.0f * mp.inv_dx * mp.inv_dx;
+  for (int a = 0; a < 3; ++a) v[a] = 0.f;
+  for (int a = 0; a < 9; ++a) nC[a] = 0.f;
 #pragma unroll 1
   for (int o = 0; o < 27; ++o) {
     const int ox = o / 9, oy = (o / 3) % 3, oz = o % 3;
-    const int I = b.base[0] + ox, Jj = b.base[1] + oy, K = b.base[2] + oz;
-    if (I < 0 || I >= G || Jj < 0 || Jj >= G || K < 0 || K >= G) continue;
-    const int64_t node = ((int64_t)K * G + Jj) * G + I;
-    const float m = g.m[node];
-    const float P[3] = {g.v[node], g.v[N + node], g.v[2 * N + node]};
-    float gv[3] = {P[0], P[1], P[2]};
-    if (m > 0.0f) {
-      const float f[3] = {g.f_ext[node], g.f_ext[N + node], g.f_ext[2 * N + node]};
-      grid_node_velocity(P, m, f, I, Jj, K, G, mp, gv);
-    }
-    const float dpos[3] = {((float)ox - b.fx[0]) * mp.dx, ((float)oy - b.fx[1]) * mp.dx, ((float)oz - b.fx[2]) * mp.dx};
+    const int id[3] = {b.base[0] + ox, b.base[1] + oy, b.base[2] + oz};
+    if (id[0] < 0 || id[0] >= G || id[1] < 0 || id[1] >= G || id[2] < 0 || id[2] >= G) continue;
     const float w = bspline_w(b.fx[0], ox) * bspline_w(b.fx[1], oy) * bspline_w(b.fx[2], oz);
-#pragma unroll
+    const float d[3] = {((float)ox - b.fx[0]) * mp.dx, ((float)oy - b.fx[1]) * mp.dx, ((float)oz - b.fx[2]) * mp.dx};
+    const int li = ((id[2] - bx.lo[2]) * bx.ext[1] + (id[1] - bx.lo[1])) * bx.ext[0] + (id[0] - bx.lo[0]);
+    const int64_t node = ((int64_t)id[2] * G + id[1]) * G + id[0];
+    const float m = stg ? 0.f : g.m[node], im = m > 0.f ? __frcp_rn(m) : 0.f;
     for (int a = 0; a < 3; ++a) {
-      nvl[a] += w * gv[a];
-#pragma unroll
-      for (int c = 0; c < 3; ++c) nC[a * 3 + c] += (w * gv[a]) * dpos[c] * s4;
+      const float gv = stg ? stg[a * nv + li]
+                           : (m > 0.f ? grid_node_component(g.v[a * N + node], im, g.f_ext[a * N + node],
+                                                            mp.gravity[a], id[a], G, mp)
+                                      : g.v[a * N + node]);
+      const float wg = w * gv;
+      v[a] += wg;
+      for (int k = 0; k < 3; ++k) nC[a * 3 + k] += wg * d[k] * s4;
     }
   }
 }
 
 // P2G payload of a particle (shared memory), one record of kQn floats per
-// particle of the chunk, in float4 groups so that the scatter reads the
-// values every lane needs as 128-bit broadcasts:
-//   [0]  mv0 mv1 mv2 mass      [4]  aff0..3      [8]  aff4..7     [12] aff8
-//   [16] base0 base1 base2 fx0 [20] fx1 fx2 pf0 pf1
-//   [24] w[0][0..2] pf2        [28] w[1][0..2]   [32] w[2][0..2]
-// (base as int bits; w the B-spline weights [axis][offset]).  A record of 36
-// floats keeps the 128-bit stores of 8 consecutive particles on distinct banks.
-enum { kQmv = 0, kQaff = 4, kQbase = 16, kQfx1 = 20, kQwx = 24, kQwy = 28, kQwz = 32, kQn = 36 };
+// particle of the chunk.  The momentum a particle gives to the stencil node
+// (ox, oy, oz), m v + A d with d the node's offset, and its weight are a sum
+// and a product over the axes, so the record holds per axis and offset o the
+// weight and that axis' share of the momentum: the scatter adds up three of
+// them per node (4 wide loads and 15 operations a particle, against 8 loads
+// and 21 operations from m v, A and the offset):
+//   [4 (3 a + o)] share0 share1 share2 weight   (a = 0: m v is in the share)
+//   [36] mass pf0 pf1 pf2                      [40] key base0 base1 base2
+// key: the index of the base node in the chunk's box (int bits), -1 when the
+// stencil leaves the grid or the chunk's box is too large; base as int bits.
+// A record of 44 floats keeps the 128-bit stores of 8 consecutive particles
+// on distinct banks.
+enum { kQmass = 36, kQkey = 40, kQn = 44 };
 
 // ---- fused substep sequence --------------------------------------------------
 // M substeps in M + 1 launches (after a prologue).  Launch s, for each chunk of
@@ -331,18 +349,43 @@ enum { kQmv = 0, kQaff = 4, kQbase = 16, kQfx1 = 20, kQwx = 24, kQwy = 28, kQwz 
 // three-kernel substep above (p2g_particle, reaction_particle, g2p_node and
 // g2p_finish on the same values).
 
-enum { kSx = 0, kSv = 3, kSC = 6, kSF = 15, kSn = 24 };  // staged particle state rows
+//
+// A CTA has one thread per particle of the chunk (four warps), which keeps the
+// particle's state in registers from the gather to the payload; the scatter
+// is by runs of one base node (see there).  Five CTA barriers per chunk.
+//
+// What bounds it: where a chunk has an SM to itself, the chain of a warp's
+// dependent instructions (some 2,500 a substep at 5 cycles each) and of the
+// trips to L2; where the SMs hold several, instruction issue.  The bytes (the
+// state of 24,576 particles and the touched nodes) move in 1 us.  So the
+// arithmetic is arranged for few instructions: no thread repeats another's
+// work, the tensor-product stencils are summed axis by axis (a node costs two
+// multiply-adds per value in the gather), the scatter adds three prepared
+// shares per node, shared memory sees no floating-point atomic (a
+// compare-and-swap loop of some 100 cycles there), the reaction's lattice box
+// arrives by asynchronous copies under the stress, statistics that a later
+// substep overwrites are not formed, and what does not depend on the previous
+// launch is read before its end.
+// One substep, before (two threads per particle, 8 warps, tile with
+// shared-memory atomics) and now, with the binning's share: 19.7 -> 14.9 us
+// (4,096 particles), 24.4 -> 21.7 us (24,576), 124 -> 87 us (196,608); the
+// 16-case batch's 11 launches 1,312 -> 700 us.  Three threads per particle (12
+// warps, one axis each) took 13-21 us at the small sizes but 116 us at 196,608
+// particles and no less than before in a batch.
+
 // bins->meta: [0] chunks, [1 + b] records in box[b], [4] chunks scattered
-// without the tile, [5 + b] buffer b holds recorded boxes not yet zeroed
+// without a tile, [5 + b] buffer b holds recorded boxes not yet zeroed
 enum { kMetaChunks = 0, kMetaRec = 1, kMetaOverflow = 4, kMetaDirty = 5 };
-constexpr int kSeqT = 256;
-constexpr int kTileFloats = (7 * kTileCap + 3) & ~3;  // keeps the next region 16-byte aligned
-// G2P: the staged node velocities use 3 * nv <= 3 * kTileCap floats of the
-// stage; the two stencil halves of a particle meet behind them (12 sums per
-// particle).  The reaction's lattice box uses 4 * nv.
-constexpr int kXchOffset = (3 * kTileCap + 3) & ~3;
-constexpr int kStageFloats = ((kXchOffset + 12 * kChunk > 4 * kTileCap ? kXchOffset + 12 * kChunk : 4 * kTileCap) + 3) & ~3;
-constexpr size_t kSeqSmem = sizeof(float) * (kTileFloats + kStageFloats + (kQn + kSn) * kChunk);
+constexpr int kSeqT = kChunk;
+constexpr int kSeqOcc = 4;          // resident CTAs per SM (by registers and by shared memory)
+// one region for the staged node velocities (G2P, 3 per node), the reaction's
+// lattice box (4 per cell) and the scatter tiles (7 per node and copy): each is
+// written after the last read of the one before it.  Four copies of the tile
+// fit for boxes of up to 243 nodes (a compact chunk of 128 particles at 8 per
+// cell has 120-220), two for 486, one for 972.
+constexpr int kStageFloats = 6816;
+static_assert(kStageFloats >= 4 * kTileCap && kStageFloats % 4 == 0, "stage holds the lattice box");
+constexpr size_t kSeqSmem = sizeof(float) * (kStageFloats + kQn * kChunk);
 
 struct SeqArgs {
   FsiParticles pt;
@@ -362,34 +405,38 @@ struct SeqArgs {
   int32_t s, M;             // launch index (0..M) and substeps in the sequence
 };
 
-// lattice coordinates of entry li of a box (two divisions)
-__device__ __forceinline__ void box_ijk(const Box& b, int li, int& i, int& j, int& k) {
-  const int e0 = b.ext[0], e01 = b.ext[0] * b.ext[1];
-  k = li / e01;
-  const int r = li - k * e01;
-  j = r / e0;
-  i = r - j * e0 + b.lo[0];
-  j += b.lo[1];
-  k += b.lo[2];
-}
+// quotient of a small non-negative integer (below 2^20) by an integer of which
+// inv is the reciprocal (small_inv): exact, as (a + 1/2) / b is at least
+// 1 / (2 b) away from an integer and the errors of inv and of the product stay
+// below 4e-7 of the quotient
+__device__ __forceinline__ float small_inv(int b) { return __fdividef(1.0f, (float)b); }
+__device__ __forceinline__ int small_div(int a, float inv) { return (int)(((float)a + 0.5f) * inv); }
 
-__device__ __forceinline__ void zero_boxes(const FsiGrid& go, const int32_t* __restrict__ rec, int nrec, int vb,
-                                           int vg) {
+// zeroes the first nq of the seven values (momentum, mass, external force) of
+// the nodes of the recorded boxes: warp w of the nw warps that share the work
+// takes the records w, w + nw, ...
+__device__ __forceinline__ void zero_boxes(const FsiGrid& go, const int32_t* __restrict__ rec, int nrec, int w, int nw,
+                                           int nq) {
   const int G = go.n;
   const int64_t N = (int64_t)G * G * G;
-  for (int r = vb; r < nrec; r += vg) {
+  for (int r = w; r < nrec; r += nw) {
     const Box bx = load_box(rec + 6 * r);
-    for (int li = threadIdx.x; li < bx.vol; li += blockDim.x) {
-      int i, j, k;
-      box_ijk(bx, li, i, j, k);
-      const int64_t node = ((int64_t)k * G + j) * G + i;
+    const int e0 = bx.ext[0], e01 = e0 * bx.ext[1];
+    const bool small = bx.vol < (1 << 20);  // the range of small_div
+    const float i0 = small_inv(max(e0, 1)), i01 = small_inv(max(e01, 1));
+    for (int li = threadIdx.x & 31; li < bx.vol; li += 32) {
+      const int k = small ? small_div(li, i01) : li / e01, q = li - k * e01;
+      const int j = small ? small_div(q, i0) : q / e0, i = q - j * e0;
+      const int64_t node = ((int64_t)(k + bx.lo[2]) * G + (j + bx.lo[1])) * G + (i + bx.lo[0]);
       go.v[node] = 0.f;
       go.v[N + node] = 0.f;
       go.v[2 * N + node] = 0.f;
       go.m[node] = 0.f;
-      go.f_ext[node] = 0.f;
-      go.f_ext[N + node] = 0.f;
-      go.f_ext[2 * N + node] = 0.f;
+      if (nq > 4) {
+        go.f_ext[node] = 0.f;
+        go.f_ext[N + node] = 0.f;
+        go.f_ext[2 * N + node] = 0.f;
+      }
     }
   }
 }
@@ -415,122 +462,146 @@ __device__ __forceinline__ FsiGrid grid_of(const SeqArgs& A, int b) {
 // zeroes every buffer with boxes left from an earlier sequence, and the
 // reaction record of the first substep
 __device__ __forceinline__ void seq_prologue_body(const SeqArgs& A, int vb, int vg) {
+  const int nw = blockDim.x >> 5;
   for (int b = 0; b < 3; ++b)
-    if (A.meta[kMetaDirty + b]) zero_boxes(grid_of(A, b), A.box + b * A.box_stride, A.meta[kMetaRec + b], vb, vg);
+    if (A.meta[kMetaDirty + b])
+      zero_boxes(grid_of(A, b), A.box + b * A.box_stride, A.meta[kMetaRec + b], vb * nw + (threadIdx.x >> 5), vg * nw, 7);
   if (A.stats && vb == 0 && threadIdx.x == 0) zero_reaction_stats(A.stats);
+}
+
+// 4-byte asynchronous copy to a shared-memory address (zero-filled when n = 0)
+__device__ __forceinline__ void copy4_async(unsigned dst, const float* src, int n) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
 }
 
 // reaction_particle() from the chunk's lattice box staged in shared memory
 // (lat[q * nv + li], q = 0..2 the force field, 3 phi; li the index in the box
-// bx, which holds every stencil node of the chunk inside the grid): the same
-// nodes, weights and summation order
-__device__ __forceinline__ void reaction_particle_staged(const float* __restrict__ lat, const Box& bx, int nv,
-                                                         const LatView& L, const FsiCouplingParams& cp,
-                                                         const BSpline& b, float Jp, float vol0, float scale,
-                                                         ReactParticle& r) {
-  float hs[3] = {0.f, 0.f, 0.f}, ps = 0.f;
-  const bool inside = b.base[0] >= 0 && b.base[1] >= 0 && b.base[2] >= 0 && b.base[0] + 2 < L.nx &&
-                      b.base[1] + 2 < L.ny && b.base[2] + 2 < L.nz;
-  const int l000 = ((b.base[2] - bx.lo[2]) * bx.ext[1] + (b.base[1] - bx.lo[1])) * bx.ext[0] + (b.base[0] - bx.lo[0]);
+// bx) for a particle whose stencil lies inside it, summed axis by axis
+__device__ __forceinline__ void reaction_particle_staged(const float* __restrict__ lat, int li, int e0, int e01, int nv,
+                                                         const FsiCouplingParams& cp, const BSpline& b, float Jp,
+                                                         float vol0, float scale, ReactParticle& r) {
+  float sum[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-  for (int ox = 0; ox < 3; ++ox)
+  for (int f = 0; f < 4; ++f) {
+    if (f == 3 && cp.kind == 0) break;
+    const float* const q = lat + li + f * nv;
 #pragma unroll
-    for (int oy = 0; oy < 3; ++oy)
+    for (int oz = 0; oz < 3; ++oz) {
+      float t = 0.f;
 #pragma unroll
-      for (int oz = 0; oz < 3; ++oz) {
-        const int I = b.base[0] + ox, Jj = b.base[1] + oy, K = b.base[2] + oz;
-        if (!inside && (I < 0 || I >= L.nx || Jj < 0 || Jj >= L.ny || K < 0 || K >= L.nz)) continue;
-        const float w = b.w[0][ox] * b.w[1][oy] * b.w[2][oz];
-        const int li = l000 + (oz * bx.ext[1] + oy) * bx.ext[0] + ox;
-        hs[0] += w * lat[li];
-        hs[1] += w * lat[nv + li];
-        hs[2] += w * lat[2 * nv + li];
-        if (cp.kind != 0) ps += w * lat[3 * nv + li];
+      for (int oy = 0; oy < 3; ++oy) {
+        const float* const x = q + oz * e01 + oy * e0;
+        t += b.w[1][oy] * (b.w[0][0] * x[0] + b.w[0][1] * x[1] + b.w[0][2] * x[2]);
       }
-  reaction_from_sums(cp, hs, ps, Jp, vol0, scale, r);
-}
-
-__device__ __forceinline__ int base_of(float x, float inv_dx) { return (int)(__fmul_rn(x, inv_dx) - 0.5f); }
-
-// the chunk's node box: min / max base node over the live threads (every
-// thread of the CTA calls this, live or not)
-__device__ __forceinline__ void box_reduce(bool live, const int nb[3], int* s_lo, int* s_hi) {
-#pragma unroll
-  for (int r = 0; r < 3; ++r) {
-    const int lo = __reduce_min_sync(0xffffffffu, live ? nb[r] : INT_MAX);
-    const int hi = __reduce_max_sync(0xffffffffu, live ? nb[r] : INT_MIN);
-    if ((threadIdx.x & 31) == 0) {
-      if (lo != INT_MAX) atomicMin(&s_lo[r], lo);
-      if (hi != INT_MIN) atomicMax(&s_hi[r], hi);
+      sum[f] += b.w[2][oz] * t;
     }
   }
+  const float hs[3] = {sum[0], sum[1], sum[2]};
+  reaction_from_sums(cp, hs, sum[3], Jp, vol0, scale, r);
 }
 
-constexpr int kRun = kChunk / (kSeqT / 32);  // particles per warp in the scatter
+// one particle's part of the reaction diagnostics
+struct ReactStats {
+  int act;              // reaction not zero
+  float pnorm, gnorm;   // norms of the particle's force and of its largest node share
+  float pf[3], gf[3];   // force of a gated particle; force given to the grid
+  float sw;             // the part of gf that reaches nodes inside the grid
+};
 
-// G2P gather of one particle over the stencil offsets o = SUB, SUB + 2, ...
-// (the two halves of the 27 nodes, one per warp of a pair) from the node
-// velocities staged in tile (box bx, nv nodes): the arithmetic of the
-// one-phase g2p_node, with the offsets, weights and offset distances known
-// per offset at compile time and the grid-range test skipped for particles
-// whose whole stencil lies inside the grid.
-template <int SUB>
-__device__ __forceinline__ void g2p_gather_half(const float* tile, int nv, const Box& bx, int G, const BSpline& b,
-                                                float dx, float s4, float* nvl, float* nC) {
-  float dp[3][3];
+__device__ __forceinline__ ReactStats reaction_stats(const ReactParticle& rp, const BSpline& b, int G) {
+  ReactStats t = {};
+  t.act = rp.act;
+  t.pnorm = rp.pnorm;
+  if (rp.gated)
+    for (int r = 0; r < 3; ++r) t.pf[r] = rp.pf[r];
+  if (rp.scatter) {
+    // the sums over the particle's nodes inside the grid factorise by axis
+    float mw = 1.f, n2 = 0.f;
+    t.sw = 1.f;
 #pragma unroll
-  for (int a = 0; a < 3; ++a)
+    for (int a = 0; a < 3; ++a) {
+      float wa = 0.f, ma = 0.f;
 #pragma unroll
-    for (int o = 0; o < 3; ++o) dp[a][o] = ((float)o - b.fx[a]) * dx;
-  const int e0 = bx.ext[0], e01 = bx.ext[0] * bx.ext[1];
-  const int li0 = ((b.base[2] - bx.lo[2]) * bx.ext[1] + (b.base[1] - bx.lo[1])) * bx.ext[0] + (b.base[0] - bx.lo[0]);
-  const bool inside = b.base[0] >= 0 && b.base[0] + 2 < G && b.base[1] >= 0 && b.base[1] + 2 < G &&
-                      b.base[2] >= 0 && b.base[2] + 2 < G;
-#pragma unroll
-  for (int o = SUB; o < 27; o += 2) {
-    const int ox = o / 9, oy = (o / 3) % 3, oz = o % 3;
-    const int I = b.base[0] + ox, Jj = b.base[1] + oy, K = b.base[2] + oz;
-    if (inside || (I >= 0 && I < G && Jj >= 0 && Jj < G && K >= 0 && K < G)) {
-      const int li = li0 + oz * e01 + oy * e0 + ox;
-      const float gv[3] = {tile[li], tile[nv + li], tile[2 * nv + li]};
-      const float dpos[3] = {dp[0][ox], dp[1][oy], dp[2][oz]};
-      const float w = b.w[0][ox] * b.w[1][oy] * b.w[2][oz];
-#pragma unroll
-      for (int q = 0; q < 3; ++q) {
-        nvl[q] += w * gv[q];
-#pragma unroll
-        for (int cc = 0; cc < 3; ++cc) nC[q * 3 + cc] += (w * gv[q]) * dpos[cc] * s4;
+      for (int o = 0; o < 3; ++o) {
+        const bool in = b.base[a] + o >= 0 && b.base[a] + o < G;
+        wa += in ? b.w[a][o] : 0.f;
+        ma = fmaxf(ma, in ? b.w[a][o] : 0.f);
       }
+      t.sw *= wa;
+      mw *= ma;
     }
+    for (int r = 0; r < 3; ++r) {
+      t.gf[r] = rp.pf[r];
+      n2 += rp.pf[r] * rp.pf[r];
+    }
+    t.gnorm = sqrtf(n2) * mw;
   }
+  return t;
 }
 
 // launch A.s of the sequence for the chunks vb, vb + vg, ... (kSeqT threads,
-// kSeqSmem bytes of dynamic shared memory)
-template <bool REACT>
+// kSeqSmem bytes of dynamic shared memory).  PDL: launched with programmatic
+// stream serialization; what is read before the wait (the chunk table, perm,
+// mass, vol0, fixed) was complete before the launch before the last one, and
+// every launch of the sequence waits for the one before it.
+template <bool REACT, bool PDL>
 __device__ __forceinline__ void mpm_seq_body(const SeqArgs& A, int vb, int vg) {
   constexpr int T = kSeqT, NW = T / 32;
-  static_assert(kSeqT == 2 * kChunk, "G2P: two warps per 32 particles, one per stencil half");
+  constexpr int NQ = REACT ? 7 : 4;  // grid values a substep writes
   extern __shared__ float4 seq_smem4[];
-  // G2P: [3][nv] node velocities; payload: [4][nv] lattice box; scatter: [7][nv] tile
-  float* const tile = reinterpret_cast<float*>(seq_smem4);  // [7][nv] scatter tile
-  float* const stg = tile + kTileFloats;                      // [3][nv] node velocities / [4][nv] lattice box
-  float* const sp = stg + kStageFloats;  // [kChunk][kQn] P2G payload
-  float* const ss = sp + kQn * kChunk;   // [kSn][kChunk] particle state
+  float* const stg = reinterpret_cast<float*>(seq_smem4);  // node velocities, then the lattice box, then the tiles
+  float* const sp = stg + kStageFloats;                    // [kChunk][kQn] P2G payload
   __shared__ int s_lo[3], s_hi[3];
+  __shared__ unsigned s_start[NW];  // bit i of word w: particle 32 w + i starts a run of one base node
   __shared__ float s_scale;
   __shared__ int s_cnt[NW];
   __shared__ float s_fmax[NW][2];
   __shared__ double s_dsum[NW][6];
+  if (PDL) {
+    // the launch's arguments into the constant caches while the previous
+    // launch still runs (a first access after the wait costs a trip to L2)
+    const int* const w = reinterpret_cast<const int*>(&A);
+#pragma unroll
+    for (int i = 0; i < (int)(sizeof(SeqArgs) / 4); i += 16) asm volatile("" ::"r"(w[i]));
+  }
   const FsiParticles& pt = A.pt;
   const FsiMpmParams& mp = A.mp;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int n = pt.n;
   const int s = A.s;
   const bool do_g2p = s > 0, do_p2g = s < A.M;
+  // the records of the last three substeps are the ones that remain: earlier ones would be overwritten
+  const bool do_stats = REACT && do_p2g && s + 3 >= A.M;
   const int bg = (s + 2) % 3, bs = s % 3, bz = (s + 1) % 3;
   const int G = A.grid[0].n;
   const int64_t N = (int64_t)G * G * G;
-  const int nch = A.meta[kMetaChunks];
+  // work items: the chunks, each cut into `split` parts where that still gives
+  // every part a CTA of its own (the substep then takes as long as one part)
+  const int nbin = A.meta[kMetaChunks];
+  int split = 1;
+  if (PDL)
+    while (split < 4 && nbin * split * 2 <= vg) split *= 2;
+  const int nch = nbin * split;
+  // this thread's particle of the CTA's first item
+  int2 ch = make_int2(0, 0);
+  int p = 0, pfixed = 0;
+  float pmass = 0.f, pvol0 = 0.f;
+  auto load_chunk = [&](int c) {
+    ch = A.chunks[c / split];
+    const int part = c % split, lo = part * ch.y / split, hi = (part + 1) * ch.y / split;
+    ch = make_int2(ch.x + lo, hi - lo);
+    if (tid < ch.y) {
+      p = A.perm[ch.x + tid];
+      pfixed = pt.fixed[p];
+      pmass = pt.mass[p];
+      pvol0 = pt.vol0[p];
+    }
+  };
+  if (vb < nch) load_chunk(vb);
+  if (PDL) {
+    griddep_wait();
+    griddep_launch();
+  }
   FsiCouplingStats* const st = REACT ? A.stats + bs : nullptr;
   if (vb == 0 && tid == 0) {
     if (s == 0) {  // the prologue zeroed every buffer
@@ -552,140 +623,143 @@ __device__ __forceinline__ void mpm_seq_body(const SeqArgs& A, int vb, int vg) {
       st->raw_area_scale = raw;
     }
   }
-  if (s >= 2) {
-    // the boxes of substep s - 2: CTAs left without a chunk (fewer chunks than
-    // CTAs) zero them, off the path of the CTAs that have one; with no idle
-    // CTA every CTA takes a share
-    const int nrec = A.meta[kMetaRec + bz], idle = vg - nch;
-    if (idle <= 0)
-      zero_boxes(grid_of(A, bz), A.box + bz * A.box_stride, nrec, vb, vg);
-    else if (vb >= nch)
-      zero_boxes(grid_of(A, bz), A.box + bz * A.box_stride, nrec, vb - nch, idle);
+  // the boxes of substep s - 2: CTAs left without a chunk (fewer chunks than
+  // CTAs) zero them, off the path of the CTAs that have one; with no idle
+  // CTA every CTA takes a share after its own chunks
+  if (vb >= nch) {
+    if (s >= 2)
+      zero_boxes(grid_of(A, bz), A.box + bz * A.box_stride, A.meta[kMetaRec + bz], (vb - nch) * NW + wid,
+                 (vg - nch) * NW, NQ);
+    return;
+  }
+  if (tid < 3) {
+    s_lo[tid] = INT_MAX;
+    s_hi[tid] = INT_MIN;
   }
 
   const float s4 = 4.0f * mp.inv_dx * mp.inv_dx;
-  const int n = pt.n;
-  int n_act = 0;
-  float pmax = 0.f, gmax = 0.f;
-  double pn[3] = {0.0, 0.0, 0.0}, gn[3] = {0.0, 0.0, 0.0};
+  if (do_stats && lane == 0) {
+    s_cnt[wid] = 0;
+    s_fmax[wid][0] = s_fmax[wid][1] = 0.f;
+#pragma unroll
+    for (int r = 0; r < 6; ++r) s_dsum[wid][r] = 0.0;
+  }
   for (int c = vb; c < nch; c += vg) {
-    __syncthreads();  // the previous chunk is done with the tile, the stages and the box
-    if (tid < 3) {
-      s_lo[tid] = INT_MAX;
-      s_hi[tid] = INT_MIN;
+    if (c != vb) {
+      load_chunk(c);
+      __syncthreads();  // the tiles of the chunk before are read
     }
-    const int2 ch = A.chunks[c];
-    int nb[3] = {0, 0, 0};  // base node of this thread's particle after the gather
-    bool nb_live = false;
-    // particle reads of the payload, issued ahead of the gather
-    const int pslot = (wid >> 1) * 32 + lane;
-    int pq = 0;
-    float pmass = 0.f, pvol0 = 0.f;
-    if (do_p2g && pslot < ch.y) {
-      pq = A.perm[ch.x + pslot];
-      pmass = pt.mass[pq];
-      pvol0 = pt.vol0[pq];
+    const bool live = tid < ch.y;
+    const Box bg_box = load_box(A.box + bg * A.box_stride + 6 * c);  // of substep s - 1 (unused at s = 0)
+    float X[3] = {0.f, 0.f, 0.f}, v[3] = {0.f, 0.f, 0.f}, C[9], F[9];
+#pragma unroll
+    for (int a = 0; a < 9; ++a) C[a] = F[a] = 0.f;
+    if (live) {
+#pragma unroll
+      for (int a = 0; a < 3; ++a) X[a] = pt.x[a * n + p];
+#pragma unroll
+      for (int a = 0; a < 9; ++a) F[a] = pt.F[(int64_t)a * n + p];
+      if (!do_g2p) {
+#pragma unroll
+        for (int a = 0; a < 3; ++a) v[a] = pt.v[a * n + p];
+#pragma unroll
+        for (int a = 0; a < 9; ++a) C[a] = pt.C[(int64_t)a * n + p];
+      }
     }
     if (do_g2p) {
       // ---- G2P of substep s - 1 from buffer bg
       const FsiGrid g = grid_of(A, bg);
-      const Box bx = load_box(A.box + bg * A.box_stride + 6 * c);
-      const bool staged = bx.vol <= kTileCap;
-      const int nv = staged ? bx.vol : 0;
-      // this lane's particle, read ahead of the staging barrier: warps 2 i and
-      // 2 i + 1 take particles 32 i .. 32 i + 31, each one half of the stencil
-      const int lp = (wid >> 1) * 32 + lane, sub = wid & 1;
-      int p = 0;
-      float X[3] = {0.f, 0.f, 0.f}, Fo[9];
-#pragma unroll
-      for (int a = 0; a < 9; ++a) Fo[a] = 0.f;
-      // the fixed flag and position, loaded with the state so that the
-      // finish does not wait on them
-      int pfixed = 0;
-      float pfx[3] = {0.f, 0.f, 0.f};
-      if (lp < ch.y) {
-        p = A.perm[ch.x + lp];
-#pragma unroll
-        for (int a = 0; a < 3; ++a) X[a] = pt.x[a * n + p];
-        if (sub == 0) {
-#pragma unroll
-          for (int a = 0; a < 9; ++a) Fo[a] = pt.F[(int64_t)a * n + p];
-          pfixed = pt.fixed[p];
-#pragma unroll
-          for (int a = 0; a < 3; ++a) pfx[a] = pt.fixed_x[a * n + p];
-        }
-      }
-      for (int li = tid; li < nv; li += T) {
-        int i, j, k;
-        box_ijk(bx, li, i, j, k);
-        const int64_t node = ((int64_t)k * G + j) * G + i;
-        const float m = g.m[node];
-        const float P[3] = {g.v[node], g.v[N + node], g.v[2 * N + node]};
-        float v[3] = {P[0], P[1], P[2]};
-        if (m > 0.0f) {
+      const Box& bx = bg_box;
+      const int nv = bx.vol <= kTileCap ? bx.vol : 0;
+      const int e0 = bx.ext[0], e01 = e0 * bx.ext[1];
+      {
+        const float i0 = small_inv(e0), i01 = small_inv(e01);
+        for (int li = tid; li < nv; li += T) {
+          const int k = small_div(li, i01), r = li - k * e01, j = small_div(r, i0), i = r - j * e0;
+          const int I = i + bx.lo[0], Jj = j + bx.lo[1], K = k + bx.lo[2];
+          const int64_t node = ((int64_t)K * G + Jj) * G + I;
+          const float m = g.m[node];
+          const float P[3] = {g.v[node], g.v[N + node], g.v[2 * N + node]};
           const float f[3] = {g.f_ext[node], g.f_ext[N + node], g.f_ext[2 * N + node]};
-          grid_node_velocity(P, m, f, i, j, k, G, mp, v);
-        }
-        stg[li] = v[0];
-        stg[nv + li] = v[1];
-        stg[2 * nv + li] = v[2];
-      }
-      __syncthreads();  // also publishes the s_lo / s_hi reset
-      float nvl[3] = {0.f, 0.f, 0.f}, nC[9] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-      BSpline b;
-      if (lp < ch.y) {
-        bspline(X, mp.inv_dx, b);
-        if (!staged) {
-          if (sub == 0) g2p_gather_global(g, mp, b, nvl, nC);
-        } else if (sub == 0) {
-          g2p_gather_half<0>(stg, nv, bx, G, b, mp.dx, s4, nvl, nC);
-        } else {
-          g2p_gather_half<1>(stg, nv, bx, G, b, mp.dx, s4, nvl, nC);
-        }
-      }
-      // the odd half's sums to the even half's lanes, through the part of
-      // the tile the staged velocities leave free
-      float* const xch = stg + kXchOffset;
-      if (sub == 1 && lp < ch.y) {
+          float u[3] = {P[0], P[1], P[2]};
+          if (m > 0.0f) {
+            const float im = __frcp_rn(m);
+            u[0] = grid_node_component(P[0], im, f[0], mp.gravity[0], I, G, mp);
+            u[1] = grid_node_component(P[1], im, f[1], mp.gravity[1], Jj, G, mp);
+            u[2] = grid_node_component(P[2], im, f[2], mp.gravity[2], K, G, mp);
+          }
 #pragma unroll
-        for (int q = 0; q < 3; ++q) xch[q * kChunk + lp] = nvl[q];
-#pragma unroll
-        for (int q = 0; q < 9; ++q) xch[(3 + q) * kChunk + lp] = nC[q];
+          for (int a = 0; a < 3; ++a) stg[a * nv + li] = u[a];
+        }
       }
       __syncthreads();
-      if (sub == 0 && lp < ch.y) {
+      if (live) {
+        BSpline b;
+        bspline(X, mp.inv_dx, b);
+        const bool inside = b.base[0] >= 0 && b.base[0] + 2 < G && b.base[1] >= 0 && b.base[1] + 2 < G &&
+                            b.base[2] >= 0 && b.base[2] + 2 < G;
+        float nC[9];
+        if (nv > 0 && inside) {
+          const float* const q =
+              stg + ((b.base[2] - bx.lo[2]) * bx.ext[1] + (b.base[1] - bx.lo[1])) * e0 + (b.base[0] - bx.lo[0]);
+          float wd[3][3];  // weight times offset from the particle
 #pragma unroll
-        for (int q = 0; q < 3; ++q) nvl[q] += xch[q * kChunk + lp];
+          for (int a = 0; a < 3; ++a)
 #pragma unroll
-        for (int q = 0; q < 9; ++q) nC[q] += xch[(3 + q) * kChunk + lp];
-        g2p_finish_f(pt, p, mp, X, nvl, nC, Fo, do_p2g ? ss : nullptr, kChunk, lp, pfixed, pfx);
+            for (int o = 0; o < 3; ++o) wd[a][o] = b.w[a][o] * (((float)o - b.fx[a]) * mp.dx);
 #pragma unroll
-        for (int r = 0; r < 3; ++r) nb[r] = base_of(X[r], mp.inv_dx);
-        nb_live = true;
+          for (int a = 0; a < 3; ++a) {
+            float n0 = 0.f, cx = 0.f, cy = 0.f, cz = 0.f;
+#pragma unroll
+            for (int oz = 0; oz < 3; ++oz) {
+              float t0 = 0.f, tx = 0.f, ty = 0.f;
+#pragma unroll
+              for (int oy = 0; oy < 3; ++oy) {
+                const float* const r = q + a * nv + oz * e01 + oy * e0;
+                const float s0 = b.w[0][0] * r[0] + b.w[0][1] * r[1] + b.w[0][2] * r[2];
+                const float s1 = wd[0][0] * r[0] + wd[0][1] * r[1] + wd[0][2] * r[2];
+                t0 += b.w[1][oy] * s0;
+                tx += b.w[1][oy] * s1;
+                ty += wd[1][oy] * s0;
+              }
+              n0 += b.w[2][oz] * t0;
+              cx += b.w[2][oz] * tx;
+              cy += b.w[2][oz] * ty;
+              cz += wd[2][oz] * t0;
+            }
+            v[a] = n0;
+            nC[a * 3] = cx * s4;
+            nC[a * 3 + 1] = cy * s4;
+            nC[a * 3 + 2] = cz * s4;
+          }
+        } else {
+          g2p_slow(nv > 0 ? stg : nullptr, nv, bx, g, mp, b, s4, v, nC);
+        }
+        float Fo[9];
+#pragma unroll
+        for (int a = 0; a < 9; ++a) Fo[a] = F[a];
+        g2p_state(pt, p, mp, pfixed != 0, X, v, nC, Fo, F);
+#pragma unroll
+        for (int a = 0; a < 9; ++a) C[a] = nC[a];
+        if (!do_p2g) pt.Jp[p] = det3(F);
       }
     } else {
       __syncthreads();  // publishes the s_lo / s_hi reset
-      if (tid < ch.y) {
-        // ---- first launch: stage the state from the particle fields
-        const int p = A.perm[ch.x + tid];
-#pragma unroll
-        for (int q = 0; q < 3; ++q) {
-          const float x = pt.x[q * n + p];
-          ss[(kSx + q) * kChunk + tid] = x;
-          ss[(kSv + q) * kChunk + tid] = pt.v[q * n + p];
-          nb[q] = base_of(x, mp.inv_dx);
-        }
-#pragma unroll
-        for (int q = 0; q < 9; ++q) {
-          ss[(kSC + q) * kChunk + tid] = pt.C[(int64_t)q * n + p];
-          ss[(kSF + q) * kChunk + tid] = pt.F[(int64_t)q * n + p];
-        }
-        nb_live = true;
-      }
     }
     if (!do_p2g) continue;
-    box_reduce(nb_live, nb, s_lo, s_hi);
-    __syncthreads();  // the state stage and the box of substep s are complete
+    // the chunk's node box: smallest and largest base node per axis
+    BSpline b;
+    bspline(X, mp.inv_dx, b);
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      const int lo = __reduce_min_sync(0xffffffffu, live ? b.base[r] : INT_MAX);
+      const int hi = __reduce_max_sync(0xffffffffu, live ? b.base[r] : INT_MIN);
+      if (lane == 0) {
+        if (lo != INT_MAX) atomicMin(&s_lo[r], lo);
+        if (hi != INT_MIN) atomicMax(&s_hi[r], hi);
+      }
+    }
+    __syncthreads();  // the box of substep s is complete, the staged velocities are read
     int32_t rec[6];
 #pragma unroll
     for (int r = 0; r < 3; ++r) {
@@ -693,202 +767,209 @@ __device__ __forceinline__ void mpm_seq_body(const SeqArgs& A, int vb, int vg) {
       rec[3 + r] = s_hi[r] == INT_MIN ? -1 : min(min(s_hi[r], G) + 2, G - 1);
     }
     const Box bx = load_box(rec);
+    const int e0 = bx.ext[0], e1 = bx.ext[1], e01 = e0 * e1;
+    // staged: the lattice box fits its region; copies: scatter tiles that fit
     const bool staged = bx.vol <= kTileCap;
     const int nv = staged ? bx.vol : 0;
+    const int stride = (NQ * nv + 3) & ~3;  // floats of a tile
+    const int copies = !staged ? 0 : (4 * stride <= kStageFloats ? 4 : (2 * stride <= kStageFloats ? 2 : (stride <= kStageFloats)));
     if (tid == 0) {
       int32_t* const out = A.box + bs * A.box_stride + 6 * c;
 #pragma unroll
       for (int r = 0; r < 6; ++r) out[r] = rec[r];
-      if (!staged) atomicAdd(A.meta + kMetaOverflow, 1);
+      if (!copies) atomicAdd(A.meta + kMetaOverflow, 1);
     }
-    // ---- P2G payload of substep s: warps of role 0 the stress and affine
-    // momentum, warps of role 1 the B-spline data and the reaction force
-    {
-      const int role = wid & 1, slot = pslot;
-      if (role == 0) {
-        if (slot < ch.y) {
-          const int p = pq;
-          P2GParticle q;
-          p2g_particle_rows(ss + kSF * kChunk, ss + kSC * kChunk, ss + kSv * kChunk, kChunk, slot, pmass, pvol0, mp,
-                            q);
-          pt.Jp[p] = q.J;
-          float* const rq = sp + slot * kQn;
-          *reinterpret_cast<float4*>(rq + kQmv) = make_float4(q.mv[0], q.mv[1], q.mv[2], q.mass);
-          *reinterpret_cast<float4*>(rq + kQaff) = make_float4(q.aff[0], q.aff[1], q.aff[2], q.aff[3]);
-          *reinterpret_cast<float4*>(rq + kQaff + 4) = make_float4(q.aff[4], q.aff[5], q.aff[6], q.aff[7]);
-          rq[kQaff + 8] = q.aff[8];
-        }
-      } else {
-        if (REACT && staged) {
-          // the chunk's lattice box (force field, phi) into shared memory, by
-          // the role-1 warps only (named barrier 1)
-          for (int li = slot; li < nv; li += T / 2) {
-            int i, j, k;
-            box_ijk(bx, li, i, j, k);
-            float h0 = 0.f, h1 = 0.f, h2 = 0.f, ph = 0.f;
-            if (i < A.L.nx && j < A.L.ny && k < A.L.nz) {
-              const int64_t cl = lat_cell(A.L, i, j, k);
-              h0 = A.hydro[cl];
-              h1 = A.hydro[A.L.pitch + cl];
-              h2 = A.hydro[2 * A.L.pitch + cl];
-              if (A.cp.kind != 0) ph = A.phi[cl];
-            }
-            stg[li] = h0;
-            stg[nv + li] = h1;
-            stg[2 * nv + li] = h2;
-            stg[3 * nv + li] = ph;
-          }
-          asm volatile("bar.sync 1, %0;" ::"n"(kSeqT / 2) : "memory");
-        }
-        if (slot < ch.y) {
-          const float X[3] = {ss[kSx * kChunk + slot], ss[(kSx + 1) * kChunk + slot], ss[(kSx + 2) * kChunk + slot]};
-          BSpline b;
-          bspline(X, mp.inv_dx, b);
-          float pf[3] = {0.f, 0.f, 0.f};
-          if (REACT) {
-            float Fp[9];
-#pragma unroll
-            for (int r = 0; r < 9; ++r) Fp[r] = ss[(kSF + r) * kChunk + slot];
-            const float J = det3(Fp);
-            ReactParticle rp;
-            if (staged)
-              reaction_particle_staged(stg, bx, nv, A.L, A.cp, b, J, pvol0, s_scale, rp);
-            else
-              reaction_particle(A.L, A.hydro, A.phi, A.cp, b, J, pvol0, s_scale, rp);
-            if (rp.act) ++n_act;
-            pmax = fmaxf(pmax, rp.pnorm);
-            if (rp.gated)
-              for (int r = 0; r < 3; ++r) pn[r] += (double)rp.pf[r];
-            if (rp.scatter)
-              for (int r = 0; r < 3; ++r) pf[r] = rp.pf[r];
-          }
-          float* const rq = sp + slot * kQn;
-          *reinterpret_cast<float4*>(rq + kQbase) =
-              make_float4(__int_as_float(b.base[0]), __int_as_float(b.base[1]), __int_as_float(b.base[2]), b.fx[0]);
-          *reinterpret_cast<float4*>(rq + kQfx1) = make_float4(b.fx[1], b.fx[2], pf[0], pf[1]);
-          *reinterpret_cast<float4*>(rq + kQwx) = make_float4(b.w[0][0], b.w[0][1], b.w[0][2], pf[2]);
-          *reinterpret_cast<float4*>(rq + kQwy) = make_float4(b.w[1][0], b.w[1][1], b.w[1][2], 0.f);
-          *reinterpret_cast<float4*>(rq + kQwz) = make_float4(b.w[2][0], b.w[2][1], b.w[2][2], 0.f);
-        }
-        // the scatter tile, free since the last flush, zeroed by the role-1
-        // warps while the role-0 warps finish the polar rotation
-        for (int i = slot; i < 7 * nv; i += T / 2) tile[i] = 0.f;
+    const float i0 = small_inv(max(e0, 1)), i01 = small_inv(max(e01, 1));
+    if (REACT && staged) {
+      // the chunk's lattice box (force field, phi), copied while the stress is computed
+      const unsigned dst = (unsigned)__cvta_generic_to_shared(stg);
+      for (int li = tid; li < nv; li += T) {
+        const int k = small_div(li, i01), r = li - k * e01, j = small_div(r, i0), i = r - j * e0;
+        const int I = i + bx.lo[0], Jj = j + bx.lo[1], K = k + bx.lo[2];
+        const int in = I < A.L.nx && Jj < A.L.ny && K < A.L.nz ? 4 : 0;
+        const int cl = in ? (K * A.L.ny + Jj) * A.L.nx + I : 0;  // below 2^31: 19 values a cell stay below 2^32
+        copy4_async(dst + 4 * li, A.hydro + cl, in);
+        copy4_async(dst + 4 * (nv + li), A.hydro + A.L.pitch + cl, in);
+        copy4_async(dst + 4 * (2 * nv + li), A.hydro + 2 * A.L.pitch + cl, in);
+        if (A.cp.kind != 0) copy4_async(dst + 4 * (3 * nv + li), A.phi + cl, in);
       }
     }
-    __syncthreads();  // payload complete, tile zeroed
-    // ---- P2G scatter of substep s into buffer bs.  Warp w takes kRun
-    // consecutive particles of the chunk, one at a time, lane o on stencil node
-    // o; particles are sorted by base node within the chunk (fsi_mpm_bin), so
-    // a run of particles with the same base is summed in registers and added
-    // to the tile with one shared-memory atomic per node value.
+    // ---- P2G payload of substep s
+    float* const rq = sp + tid * kQn;
+    float J = 1.f;
+    if (live) {
+      P2GParticle q;
+      p2g_particle_state(F, C, v, pmass, pvol0, mp, q);
+      J = q.J;
+      pt.Jp[p] = J;
+#pragma unroll
+      for (int a = 0; a < 3; ++a)
+#pragma unroll
+        for (int o = 0; o < 3; ++o) {
+          const float d = ((float)o - b.fx[a]) * mp.dx;
+          float t[3];
+#pragma unroll
+          for (int r = 0; r < 3; ++r) t[r] = a == 0 ? q.mv[r] + q.aff[r * 3] * d : q.aff[r * 3 + a] * d;
+          *reinterpret_cast<float4*>(rq + 4 * (3 * a + o)) = make_float4(t[0], t[1], t[2], b.w[a][o]);
+        }
+    }
+    if (REACT && staged) {
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      __syncthreads();
+    }
+    ReactStats st_add = {};
+    if (live) {
+      const bool inside = b.base[0] >= 0 && b.base[0] + 2 < G && b.base[1] >= 0 && b.base[1] + 2 < G &&
+                          b.base[2] >= 0 && b.base[2] + 2 < G;
+      const int li = ((b.base[2] - bx.lo[2]) * e1 + (b.base[1] - bx.lo[1])) * e0 + (b.base[0] - bx.lo[0]);
+      float pf[3] = {0.f, 0.f, 0.f};
+      if (REACT) {
+        ReactParticle rp;
+        if (staged && inside)
+          reaction_particle_staged(stg, li, e0, e01, nv, A.cp, b, J, pvol0, s_scale, rp);
+        else
+          reaction_particle(A.L, A.hydro, A.phi, A.cp, b, J, pvol0, s_scale, rp);
+        if (rp.scatter)
+          for (int r = 0; r < 3; ++r) pf[r] = rp.pf[r];
+        if (do_stats) st_add = reaction_stats(rp, b, G);
+      }
+      *reinterpret_cast<float4*>(rq + kQmass) = make_float4(pmass, pf[0], pf[1], pf[2]);
+      *reinterpret_cast<int4*>(rq + kQkey) = make_int4(copies && inside ? li : -1, b.base[0], b.base[1], b.base[2]);
+    }
+    if (do_stats) {
+      // the warp's part of the diagnostics reductions (penalty.py:202-240, moving_boundary.py:312-374)
+      const int na = __reduce_add_sync(0xffffffffu, (unsigned)st_add.act);
+      const float pm = warp_max(st_add.pnorm), gm = warp_max(st_add.gnorm);
+      double r6[6];
+#pragma unroll
+      for (int r = 0; r < 3; ++r) {
+        r6[r] = warp_sum_d((double)st_add.pf[r]);
+        r6[3 + r] = warp_sum_d((double)st_add.gf[r] * (double)st_add.sw);
+      }
+      if (lane == 0) {
+        s_cnt[wid] += na;
+        s_fmax[wid][0] = fmaxf(s_fmax[wid][0], pm);
+        s_fmax[wid][1] = fmaxf(s_fmax[wid][1], gm);
+#pragma unroll
+        for (int r = 0; r < 6; ++r) s_dsum[wid][r] += r6[r];
+      }
+    }
+    {
+      const int q0 = __shfl_up_sync(0xffffffffu, b.base[0], 1), q1 = __shfl_up_sync(0xffffffffu, b.base[1], 1),
+                q2 = __shfl_up_sync(0xffffffffu, b.base[2], 1);
+      const unsigned start = __ballot_sync(
+          0xffffffffu, live && (lane == 0 || q0 != b.base[0] || q1 != b.base[1] || q2 != b.base[2]));
+      if (lane == 0) s_start[wid] = start;
+    }
+    __syncthreads();  // payload complete, the lattice box is read
+    if (tid < 3) {
+      s_lo[tid] = INT_MAX;
+      s_hi[tid] = INT_MIN;
+    }
+    // ---- P2G scatter of substep s into buffer bs, in two steps without
+    // floating-point atomics in shared memory (each is a compare-and-swap loop
+    // of some 100 cycles).  Particles are sorted by base node within the chunk
+    // (fsi_mpm_bin), so they come in runs of one base node.
+    // (1) Each warp sums its runs, one particle at a time, lane o on stencil
+    // node o (lanes 27-31 are not used), and adds a run's 27 x 7 sums to its own copy of the tile.  With
+    // fewer copies than warps the warps take turns.
     const FsiGrid g = grid_of(A, bs);
     float* const dst[7] = {g.v, g.v + N, g.v + 2 * N, g.m, g.f_ext, g.f_ext + N, g.f_ext + 2 * N};
     {
-      constexpr int NQ = REACT ? 7 : 4;
       const int ox = lane / 9, oy = (lane / 3) % 3, oz = lane % 3;
-      const float dox = (float)ox, doy = (float)oy, doz = (float)oz;
-      float gsum[3] = {0.f, 0.f, 0.f}, gm2 = 0.f;
-      float acc[NQ];
+      // lanes 27-31 read offset 2 of the x axis and are not used
+      const int q0 = 4 * min(ox, 2), q1 = 12 + 4 * oy, q2 = 24 + 4 * oz;
+      const int node_off = oz * e01 + oy * e0 + ox;
+      const int words = (ch.y + 31) >> 5;            // words of 32 particles that hold any
+      const int share = words <= 1 ? NW : (words == 2 ? NW / 2 : 1);  // warps that share a word's runs
+      const int word = wid / share, mine = wid % share;
+      float* const tile = stg + (copies ? wid % copies : 0) * stride;
+      if (wid < copies) {
+        for (int i = lane; i < stride / 4; i += 32) reinterpret_cast<float4*>(tile)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        __syncwarp();
+      }
+      const int rounds = copies ? NW / copies : 1;
+      for (int round = 0; round < rounds; ++round) {
+        if (round > 0) __syncthreads();
+        if (copies && wid / copies != round) continue;
+        unsigned m = word < words ? s_start[word] : 0u;
+        const int last = min(word * 32 + 32, ch.y);
+        for (int turn = 0; m; turn = turn + 1 == share ? 0 : turn + 1) {
+          const int first = word * 32 + __ffs(m) - 1;
+          m &= m - 1;
+          const int end = m ? word * 32 + __ffs(m) - 1 : last;
+          if (turn != mine) continue;
+          const float* rp = sp + first * kQn;
+          const int4 head = *reinterpret_cast<const int4*>(rp + kQkey);
+          const int key = head.x;
+          // the run's sums continue those of the tile (0 where it goes to the grid)
+          float* const t = tile + (key >= 0 && lane < 27 ? key + node_off : 0);
+          float acc[NQ];
 #pragma unroll
-      for (int q = 0; q < NQ; ++q) acc[q] = 0.f;
-      int cb0 = INT_MIN, cb1 = 0, cb2 = 0;  // base of the run (warp-uniform)
-      // adds the run's sums of this lane's node to the tile (or the grid)
-      auto flush_run = [&]() {
-        const int I = cb0 + ox, Jj = cb1 + oy, K = cb2 + oz;
-        if (lane < 27 && I >= 0 && I < G && Jj >= 0 && Jj < G && K >= 0 && K < G) {
-          if (staged) {
-            const int li = ((K - bx.lo[2]) * bx.ext[1] + (Jj - bx.lo[1])) * bx.ext[0] + (I - bx.lo[0]);
-#pragma unroll
-            for (int q = 0; q < NQ; ++q)
-              if (acc[q] != 0.f) atomicAdd(&tile[q * nv + li], acc[q]);
-          } else {
-            const int64_t node = ((int64_t)K * G + Jj) * G + I;
-#pragma unroll
-            for (int q = 0; q < NQ; ++q)
-              if (acc[q] != 0.f) atomicAdd(dst[q] + node, acc[q]);
+          for (int q = 0; q < NQ; ++q) acc[q] = key >= 0 && lane < 27 ? t[q * nv] : 0.f;
+#pragma unroll 2
+          for (int lp = first; lp < end; ++lp, rp += kQn) {
+            const float4 x4 = *reinterpret_cast<const float4*>(rp + q0);
+            const float4 y4 = *reinterpret_cast<const float4*>(rp + q1);
+            const float4 z4 = *reinterpret_cast<const float4*>(rp + q2);
+            const float4 f4 = *reinterpret_cast<const float4*>(rp + kQmass);
+            const float w = x4.w * y4.w * z4.w;
+            acc[0] += w * (x4.x + y4.x + z4.x);
+            acc[1] += w * (x4.y + y4.y + z4.y);
+            acc[2] += w * (x4.z + y4.z + z4.z);
+            acc[3] += w * f4.x;
+            if (REACT) {
+              acc[NQ - 3] += w * f4.y;
+              acc[NQ - 2] += w * f4.z;
+              acc[NQ - 1] += w * f4.w;
+            }
           }
-        }
+          if (key >= 0) {
+            if (lane < 27) {
 #pragma unroll
-        for (int q = 0; q < NQ; ++q) acc[q] = 0.f;
-      };
-      const int p1 = min(wid * kRun + kRun, ch.y);
-      for (int lp = wid * kRun; lp < p1; ++lp) {
-        const float* const rq = sp + lp * kQn;
-        const float4 q4 = *reinterpret_cast<const float4*>(rq + kQbase);
-        const int b0 = __float_as_int(q4.x), b1 = __float_as_int(q4.y), b2 = __float_as_int(q4.z);
-        if (b0 != cb0 || b1 != cb1 || b2 != cb2) {
-          if (cb0 != INT_MIN) flush_run();
-          cb0 = b0;
-          cb1 = b1;
-          cb2 = b2;
-        }
-        if (lane < 27) {
-          // weights of bspline() (staged by the payload) and offsets as in p2g_node()
-          const float4 q5 = *reinterpret_cast<const float4*>(rq + kQfx1);
-          const float w = rq[kQwx + ox] * rq[kQwy + oy] * rq[kQwz + oz];
-          const float dpos[3] = {(dox - q4.w) * mp.dx, (doy - q5.x) * mp.dx, (doz - q5.y) * mp.dx};
-          const float4 m4 = *reinterpret_cast<const float4*>(rq + kQmv);
-          const float4 a0 = *reinterpret_cast<const float4*>(rq + kQaff);
-          const float4 a1 = *reinterpret_cast<const float4*>(rq + kQaff + 4);
-          const float a8 = rq[kQaff + 8];
-          const float mv[3] = {m4.x, m4.y, m4.z};
-          const float aff[9] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w, a8};
+              for (int q = 0; q < NQ; ++q) t[q * nv] = acc[q];
+            }
+            __syncwarp();  // the next run may share nodes
+          } else if (lane < 27) {
+            // a stencil that leaves the grid, or a box too large: to the grid
+            const int I = head.y + ox, Jj = head.z + oy, K = head.w + oz;
+            if (I >= 0 && I < G && Jj >= 0 && Jj < G && K >= 0 && K < G) {
+              const int64_t node = ((int64_t)K * G + Jj) * G + I;
 #pragma unroll
-          for (int q = 0; q < 3; ++q)
-            acc[q] += w * (mv[q] + (aff[3 * q] * dpos[0] + aff[3 * q + 1] * dpos[1] + aff[3 * q + 2] * dpos[2]));
-          acc[3] += w * m4.w;
-          if (REACT) {
-            const float f0 = q5.z, f1 = q5.w, f2 = rq[kQwx + 3];
-            if (f0 != 0.f || f1 != 0.f || f2 != 0.f) {
-              const float v4 = w * f0, v5 = w * f1, v6 = w * f2;
-              acc[NQ - 3] += v4;
-              acc[NQ - 2] += v5;
-              acc[NQ - 1] += v6;
-              gsum[0] += v4;
-              gsum[1] += v5;
-              gsum[2] += v6;
-              gm2 = fmaxf(gm2, v4 * v4 + v5 * v5 + v6 * v6);
+              for (int q = 0; q < NQ; ++q)
+                if (acc[q] != 0.f) atomicAdd(dst[q] + node, acc[q]);
             }
           }
         }
       }
-      if (cb0 != INT_MIN) flush_run();
-      if (REACT) {
-#pragma unroll
-        for (int q = 0; q < 3; ++q) gn[q] += (double)gsum[q];
-        gmax = fmaxf(gmax, sqrtf(gm2));
-      }
     }
     __syncthreads();
-    for (int li = tid; li < nv; li += T) {
-      int i, j, k;
-      box_ijk(bx, li, i, j, k);
-      const int64_t node = ((int64_t)k * G + j) * G + i;
+    // (2) One thread per node of the box adds the copies' values and gives
+    // each to the grid with one global atomic.
+    for (int li = tid; copies && li < nv; li += T) {
+      const int k = small_div(li, i01), r = li - k * e01, j = small_div(r, i0), i = r - j * e0;
+      const int64_t node = ((int64_t)(k + bx.lo[2]) * G + (j + bx.lo[1])) * G + (i + bx.lo[0]);
+      const float* const t = stg + li;
+      float val[NQ];
 #pragma unroll
-      for (int q = 0; q < 7; ++q) {
-        const float v = tile[q * nv + li];
-        if (v != 0.f) atomicAdd(dst[q] + node, v);
+      for (int q = 0; q < NQ; ++q) val[q] = t[q * nv];
+      if (copies > 1) {
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) val[q] += t[stride + q * nv];
       }
+      if (copies > 2) {
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) val[q] += t[2 * stride + q * nv] + t[3 * stride + q * nv];
+      }
+#pragma unroll
+      for (int q = 0; q < NQ; ++q)
+        if (val[q] != 0.f) atomicAdd(dst[q] + node, val[q]);
     }
   }
-  if (REACT && do_p2g) {
-    // diagnostics reductions (penalty.py:202-240, moving_boundary.py:312-374):
-    // warp, then CTA, then one global atomic per CTA and quantity
-    const int na = __reduce_add_sync(0xffffffffu, (unsigned)n_act);
-    const float pm = warp_max(pmax), gm = warp_max(gmax);
-    double r6[6];
-#pragma unroll
-    for (int r = 0; r < 3; ++r) {
-      r6[r] = warp_sum_d(pn[r]);
-      r6[3 + r] = warp_sum_d(gn[r]);
-    }
-    if (lane == 0) {
-      s_cnt[wid] = na;
-      s_fmax[wid][0] = pm;
-      s_fmax[wid][1] = gm;
-#pragma unroll
-      for (int r = 0; r < 6; ++r) s_dsum[wid][r] = r6[r];
-    }
+  if (vg <= nch && s >= 2)
+    zero_boxes(grid_of(A, bz), A.box + bz * A.box_stride, A.meta[kMetaRec + bz], vb * NW + wid, vg * NW, NQ);
+  if (do_stats) {
+    // the CTA's part: one global atomic per CTA and quantity
     __syncthreads();
     if (tid == 0) {
       int ca = 0;
@@ -918,10 +999,8 @@ __global__ __launch_bounds__(kSeqT) void k_mpm_seq_prologue(const __grid_constan
 }
 
 template <bool REACT>
-__global__ __launch_bounds__(kSeqT, 2) void k_mpm_seq(const __grid_constant__ SeqArgs A) {
-  griddep_wait();
-  griddep_launch();
-  mpm_seq_body<REACT>(A, blockIdx.x, gridDim.x);
+__global__ __launch_bounds__(kSeqT, kSeqOcc) void k_mpm_seq(const __grid_constant__ SeqArgs A) {
+  mpm_seq_body<REACT, true>(A, blockIdx.x, gridDim.x);
 }
 
 __global__ void k_grid_velocity(FsiGrid g, FsiMpmParams mp, float* __restrict__ out) {
@@ -1164,13 +1243,13 @@ __global__ __launch_bounds__(kSeqT) void k_batch_mpm_seq_prologue(const FsiBatch
   seq_prologue_body(A, blockIdx.x, gridDim.x);
 }
 
-__global__ __launch_bounds__(kSeqT, 2) void k_batch_mpm_seq(const FsiBatchCase* __restrict__ cases, int s, int M) {
+__global__ __launch_bounds__(kSeqT, kSeqOcc) void k_batch_mpm_seq(const FsiBatchCase* __restrict__ cases, int s, int M) {
   __shared__ SeqArgs A;
   const FsiBatchCase& bc = cases[blockIdx.y];
   if (!bc.active) return;
   if (threadIdx.x == 0) load_batch_seq(bc, s, M, &A);
   __syncthreads();
-  mpm_seq_body<true>(A, blockIdx.x, gridDim.x);
+  mpm_seq_body<true, false>(A, blockIdx.x, gridDim.x);
 }
 
 __global__ __launch_bounds__(kSortT) void k_batch_bin_sort(const FsiBatchCase* __restrict__ cases) {

@@ -79,19 +79,12 @@ struct P2GParticle {
   float aff[9];  // -dt vol0 P F^T inv_dx^2 + m C (solid.py:239: no factor 4)
 };
 
-// the particle's state read from rows of stride `ld` (global SoA fields with
-// ld = n, or a shared-memory stage with ld = chunk size), column `col`
-__device__ __forceinline__ void p2g_particle_rows(const float* __restrict__ Frow, const float* __restrict__ Crow,
-                                                  const float* __restrict__ vrow, int64_t ld, int col, float mass,
-                                                  float vol0, const FsiMpmParams& mp, P2GParticle& q) {
-  float Fp[9], Cp[9];
+// from the particle's state in registers
+__device__ __forceinline__ void p2g_particle_state(const float Fp[9], const float Cp[9], const float v[3], float mass,
+                                                   float vol0, const FsiMpmParams& mp, P2GParticle& q) {
   double Fd[9], Rd[9];
 #pragma unroll
-  for (int a = 0; a < 9; ++a) {
-    Fp[a] = Frow[a * ld + col];
-    Cp[a] = Crow[a * ld + col];
-    Fd[a] = (double)Fp[a];
-  }
+  for (int a = 0; a < 9; ++a) Fd[a] = (double)Fp[a];
   polar_rotation_d(Fd, Rd);
   const float c00 = Fp[4] * Fp[8] - Fp[5] * Fp[7];
   const float c01 = Fp[3] * Fp[8] - Fp[5] * Fp[6];
@@ -125,11 +118,20 @@ __device__ __forceinline__ void p2g_particle_rows(const float* __restrict__ Frow
       q.aff[i * 3 + j] = pf * mp.inv_dx * mp.inv_dx + mass * Cp[i * 3 + j];
     }
 #pragma unroll
-  for (int a = 0; a < 3; ++a) q.mv[a] = mass * vrow[a * ld + col];
+  for (int a = 0; a < 3; ++a) q.mv[a] = mass * v[a];
 }
 
 __device__ __forceinline__ void p2g_particle(const FsiParticles& pt, int p, const FsiMpmParams& mp, P2GParticle& q) {
-  p2g_particle_rows(pt.F, pt.C, pt.v, pt.n, p, pt.mass[p], pt.vol0[p], mp, q);
+  const int64_t n = pt.n;
+  float F[9], C[9], v[3];
+#pragma unroll
+  for (int a = 0; a < 9; ++a) {
+    F[a] = pt.F[a * n + p];
+    C[a] = pt.C[a * n + p];
+  }
+#pragma unroll
+  for (int a = 0; a < 3; ++a) v[a] = pt.v[a * n + p];
+  p2g_particle_state(F, C, v, pt.mass[p], pt.vol0[p], mp, q);
 }
 
 // momentum carried to the node at stencil offset (ox, oy, oz)
@@ -230,24 +232,14 @@ __device__ __forceinline__ float det3(const float (&M)[9]) {
   return M[0] * (M[4] * M[8] - M[5] * M[7]) - M[1] * (M[3] * M[8] - M[5] * M[6]) + M[2] * (M[3] * M[7] - M[4] * M[6]);
 }
 
-// advect, clamp, update F and apply the step-112 controls, then store
-// (solid.py:261-315); nv and nC are the gathered velocity and affine matrix.
-// With a stage (rows x 3, v 3, C 9, F 9 of stride ld, column col) the new
-// state is also written there.  fixed_pre / fx_pre: the particle's fixed flag
-// and fixed position when the caller loaded them ahead (-1 / null: loaded
-// here).
-// Fo: the particle's deformation gradient before the substep
-__device__ __forceinline__ void g2p_finish_f(const FsiParticles& pt, int p, const FsiMpmParams& mp, float X[3],
-                                             const float nv[3], float nC[9], const float Fo[9],
-                                             float* stage = nullptr, int ld = 0, int col = 0, int fixed_pre = -1,
-                                             const float* fx_pre = nullptr) {
+// advect, clamp, update F and apply the step-112 controls, then store x, v, C
+// and F (solid.py:261-315).  X: position, v: gathered velocity, nC: affine
+// matrix (all updated); Fo, Fn: deformation gradient before and after.
+__device__ __forceinline__ void g2p_state(const FsiParticles& pt, int p, const FsiMpmParams& mp, bool fixed, float X[3],
+                                          float v[3], float nC[9], const float Fo[9], float Fn[9]) {
   const int n = pt.n;
-  float v[3];
 #pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    v[a] = nv[a];
-    X[a] += mp.dt * nv[a];
-  }
+  for (int a = 0; a < 3; ++a) X[a] += mp.dt * v[a];
   // clamp_particle_to_domain (solid.py:114-124)
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
@@ -260,7 +252,6 @@ __device__ __forceinline__ void g2p_finish_f(const FsiParticles& pt, int p, cons
       if (v[a] > 0.f) v[a] = 0.f;
     }
   }
-  float Fn[9];
 #pragma unroll
   for (int a = 0; a < 3; ++a)
 #pragma unroll
@@ -270,7 +261,6 @@ __device__ __forceinline__ void g2p_finish_f(const FsiParticles& pt, int p, cons
       for (int k = 0; k < 3; ++k) acc += ((a == k ? 1.0f : 0.0f) + mp.dt * nC[a * 3 + k]) * Fo[k * 3 + c];
       Fn[a * 3 + c] = acc;
     }
-  float J = det3(Fn);
   // apply_step112_dynamics_controls (solid.py:301-315)
   if (mp.damping > 0.f) {
     const float d = fmaxf(0.0f, 1.0f - mp.damping * mp.dt);
@@ -278,7 +268,7 @@ __device__ __forceinline__ void g2p_finish_f(const FsiParticles& pt, int p, cons
     for (int a = 0; a < 3; ++a) v[a] *= d;
   }
   if (mp.lock_z) {
-    X[2] = fx_pre ? fx_pre[2] : pt.fixed_x[2 * n + p];
+    X[2] = pt.fixed_x[2 * n + p];
     v[2] = 0.f;
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
@@ -288,12 +278,11 @@ __device__ __forceinline__ void g2p_finish_f(const FsiParticles& pt, int p, cons
       Fn[d * 3 + 2] = 0.f;
     }
     Fn[8] = 1.0f;
-    J = det3(Fn);
   }
-  if (fixed_pre >= 0 ? fixed_pre != 0 : pt.fixed[p] != 0) {
+  if (fixed) {
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-      X[a] = fx_pre ? fx_pre[a] : pt.fixed_x[a * n + p];
+      X[a] = pt.fixed_x[a * n + p];
       v[a] = 0.f;
     }
 #pragma unroll
@@ -301,7 +290,6 @@ __device__ __forceinline__ void g2p_finish_f(const FsiParticles& pt, int p, cons
       nC[a] = 0.f;
       Fn[a] = (a % 4 == 0) ? 1.0f : 0.0f;
     }
-    J = 1.0f;
   }
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
@@ -313,27 +301,15 @@ __device__ __forceinline__ void g2p_finish_f(const FsiParticles& pt, int p, cons
     pt.C[(int64_t)a * n + p] = nC[a];
     pt.F[(int64_t)a * n + p] = Fn[a];
   }
-  pt.Jp[p] = J;
-  if (stage) {
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      stage[a * ld + col] = X[a];
-      stage[(3 + a) * ld + col] = v[a];
-    }
-#pragma unroll
-    for (int a = 0; a < 9; ++a) {
-      stage[(6 + a) * ld + col] = nC[a];
-      stage[(15 + a) * ld + col] = Fn[a];
-    }
-  }
 }
 
 __device__ __forceinline__ void g2p_finish(const FsiParticles& pt, int p, const FsiMpmParams& mp, float X[3],
                                            const float nv[3], float nC[9]) {
-  float Fo[9];
+  float Fo[9], Fn[9], v[3] = {nv[0], nv[1], nv[2]};
 #pragma unroll
   for (int a = 0; a < 9; ++a) Fo[a] = pt.F[(int64_t)a * pt.n + p];
-  g2p_finish_f(pt, p, mp, X, nv, nC, Fo);
+  g2p_state(pt, p, mp, pt.fixed[p] != 0, X, v, nC, Fo, Fn);
+  pt.Jp[p] = det3(Fn);
 }
 
 // one gathered node's contribution to the particle velocity and affine matrix
