@@ -205,6 +205,13 @@ int fsi_lbm_to_natural(const FsiLbmState* s, void* stream);
  * collision (398-413) -> AA streaming with static or moving half-way
  * bounce-back and momentum-exchange link forces (431-440 / 488-536). */
 int fsi_lbm_substep(const FsiLbmState* s, const FsiLbmParams* p, const FsiStepCtl* ctl, void* stream);
+
+/* n moving-boundary substeps in a row (FSI_MODE_MOVING_BB, optionally
+ * FSI_MODE_SUBCYCLED; no per-direction reductions, no penalty force): n calls of
+ * fsi_lbm_substep with parity and pp flipped and bc_pending set between them,
+ * without a return to the caller's language after each. */
+int fsi_lbm_substeps(const FsiLbmState* s, const FsiLbmParams* p, const FsiStepCtl* ctl, int32_t n, void* stream);
+
 /* Under semantics 4-9 fsi_lbm_substep launches one more small kernel after the
  * step: the clear of the repair step counters and, under 8 and 9, the outlet
  * flux controller (update_open_boundary_plane_flux_controller, fluid.py:1141-1263)

@@ -177,6 +177,7 @@ SIGNATURES = {
     "fsi_lbm_set_solid": [_P(FsiLbmState), c_p, c_p],
     "fsi_lbm_to_natural": [_P(FsiLbmState), c_p],
     "fsi_lbm_substep": [_P(FsiLbmState), _P(FsiLbmParams), _P(FsiStepCtl), c_p],
+    "fsi_lbm_substeps": [_P(FsiLbmState), _P(FsiLbmParams), _P(FsiStepCtl), c_i32, c_p],
     "fsi_ob_controller_update": [_P(FsiLbmState), _P(FsiLbmParams), c_p, c_p, c_p],
     "fsi_lbm_flush_bc": [_P(FsiLbmState), _P(FsiLbmParams), _P(FsiStepCtl), c_p],
     "fsi_mask_rebuild": [_P(FsiLbmState), _P(FsiLbmParams), _P(FsiStepCtl), c_f32, c_p],

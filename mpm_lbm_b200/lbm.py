@@ -413,6 +413,31 @@ class LBMFluid3D:
         self._fused_accumulation = bool(mode & FSI_MODE_SUBCYCLED)
         self._substep(mode)
 
+    def step_moving_bounceback_run(self, n):
+        """n step_moving_bounceback() without per-direction reductions, each
+        followed by accumulate_moving_boundary_force_sample() when the subcycle
+        accumulator is open, through one call of the library (fsi_lbm_substeps)."""
+        if n <= 0:
+            return
+        if self.tau_f is None:
+            raise RuntimeError("init_simulation() must run before stepping")
+        mode = FSI_MODE_MOVING_BB | (FSI_MODE_SUBCYCLED if self._accumulating else 0)
+        self._sync_params()
+        ctl = self._ctl(mode)
+        call("fsi_lbm_substeps", ctypes.byref(self.state), ctypes.byref(self.params), ctypes.byref(ctl), int(n),
+             self._stream())
+        self.last_pp = (self.pp + n - 1) & 1
+        self.pp ^= n & 1
+        self.parity ^= n & 1
+        self.bc_pending = bool(self.bc_x_left or self.bc_x_right)
+        self.steps += n
+        self._version += n
+        self._penalty = None
+        self._hydro_src = self.last_pp
+        self._fused_accumulation = self._accumulating
+        if self._accumulating:
+            self._sample_count += n
+
     def flush_open_boundary(self):
         if self.bc_pending:
             call("fsi_lbm_flush_bc", ctypes.byref(self.state), ctypes.byref(self.params),
