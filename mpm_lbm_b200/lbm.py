@@ -21,7 +21,7 @@ import torch
 
 from . import _lib
 from ._lib import (FSI_CELL_OVERRIDE, FSI_CELL_SOLID, FSI_MODE_DIRSTATS, FSI_MODE_MOVING_BB, FSI_MODE_PENALTY,
-                   FSI_MODE_SUBCYCLED, FsiLbmDiag, FsiLbmParams, FsiLbmState, FsiStepCtl, call, ptr, stream_handle)
+                   FSI_MODE_SUBCYCLED, FSI_TUNE_LBM_OCC3, FSI_TUNE_LBM_OCC3_PF, FSI_TUNE_LBM_OCC4, FsiLbmDiag, FsiLbmParams, FsiLbmState, FsiStepCtl, call, ptr, stream_handle)
 from .config import (KERNEL_OPEN_BOUNDARY_CODES, LEGACY_EXTERNAL_SOLVER_RELAXATION_PARAMETER,
                      STANDARD_LATTICE_KINEMATIC_VISCOSITY, LBMConfig, tau_from_lattice_kinematic_viscosity,
                      tau_from_legacy_external_solver_parameter)
@@ -46,6 +46,23 @@ def relaxation_rates(tau: float, collision: str = "mrt"):
     s_v = 1.0 / tau
     s_o = s_v if collision == "bgk" else 8.0 * (2.0 - s_v) / (8.0 - s_v)
     return s_v, s_o
+
+
+L2_BYTES = 126e6
+
+
+def default_tune(cells: int, nx: int, fp16: bool, open_faces: bool) -> int:
+    """Launch variant of the step kernel where nobody has timed them.  us per step, 3 CTAs / 4 CTAs / 3 CTAs with the
+    L2 prefetch: populations beyond the L2 cache and rows that start a 32-cell block, so that a prefetched line is one
+    warp's: 57.7 / 59.1 / 55.0 (128^3), 144.2 / 146.9 / 132.7 (192x176x160), FP16 149.7 / 143.0 / 139.9; without
+    such rows the prefetch costs more than it gives, 89.8 / 86.5 / 91.7 (150x130x140, open faces).  Below, the fourth
+    CTA pays where a cell takes more instructions, FP16 storage (24.7 / 24.2, 96^3) or open faces (55.0 / 53.1,
+    192x96x96), unless the lattice is a wave or less of CTAs (64x40x40: 7.1 / 7.6); else 20.0 / 20.3 (96^3)."""
+    if 19 * cells * (2 if fp16 else 4) > L2_BYTES and nx % 32 == 0:
+        return FSI_TUNE_LBM_OCC3_PF
+    if (fp16 or open_faces) and cells > 200_000:
+        return FSI_TUNE_LBM_OCC4
+    return FSI_TUNE_LBM_OCC3
 
 
 class LBMFluid3D:
@@ -118,7 +135,8 @@ class LBMFluid3D:
         self._readout_version = -1
         self._old_equals_solid = False
         self.dirstats_enabled = True
-        self.tune = 0  # FSI_TUNE_LBM_* launch variant (mpm_lbm_b200.autotune picks it)
+        # FSI_TUNE_LBM_* launch variant (mpm_lbm_b200.autotune times them on a case)
+        self.tune = default_tune(n, self.nx, self.fp16, bool(self.bc_x_left or self.bc_x_right))
         self.tau_f = None
         self._sync_params()
         self._make_fields()
