@@ -2989,12 +2989,6 @@ extern "C" int fsi_mask_rebuild_static_scratch(const FsiLbmState* s, const FsiLb
 // its case's lattice descriptors in shared memory once.
 namespace fsi {
 
-__device__ __forceinline__ void copy_words(void* dst, const void* src, int bytes, int tid, int nt) {
-  const int* s = static_cast<const int*>(src);
-  int* d = static_cast<int*>(dst);
-  for (int i = tid; i < bytes / 4; i += nt) d[i] = s[i];
-}
-
 // stage the lattice part of a batch case (state, params, step control, and the
 // MRT rates when with_k) in shared memory; returns false for an inactive slot
 __device__ __forceinline__ bool stage_case(const FsiBatchCase& bc, Case& sc, bool with_k) {
@@ -3125,9 +3119,8 @@ int check_batch(const FsiBatchCase* cases, const FsiBatchDims* d) {
   return FSI_OK;
 }
 
-static inline unsigned batch_x(int64_t work, int threads, int cap) {
-  const int64_t b = (work + threads - 1) / threads;
-  return (unsigned)std::max<int64_t>(1, std::min<int64_t>(b, cap));
+static inline unsigned batch_x(int64_t work, int cap) {
+  return (unsigned)std::max<int64_t>(1, std::min<int64_t>(work, cap));
 }
 
 }  // namespace fsi
@@ -3138,16 +3131,16 @@ extern "C" int fsi_batch_lbm_substep(FsiBatchCase* cases, const FsiBatchDims* d,
   cudaStream_t st = (cudaStream_t)stream;
   k_batch_ctl<<<d->n_cases, 32, 0, st>>>(cases, kBatchLbmPre);
   if ((rc = launch_check("k_batch_ctl"))) return rc;
-  // one CTA per tile of the largest case; CTAs past a smaller case's tiles exit at once
+  // one CTA per one to four tiles of the largest case; CTAs past a smaller case's tiles exit at once
   if (d->lbm_tune == FSI_TUNE_LBM_PAIR) {
     // max_lbm_tiles counts 32 x 8 x 1 tiles; a 64 x 4 tile covers as many cells
-    const dim3 grid(batch_x((int64_t)d->max_lbm_tiles + 64, 1, 1 << 20), d->n_cases);
+    const dim3 grid(batch_x((int64_t)d->max_lbm_tiles + 64, 1 << 20), d->n_cases);
     if (d->store_fp16)
       k_batch_lbm_step2<true><<<grid, dim3(32, 4), 0, st>>>(cases);
     else
       k_batch_lbm_step2<false><<<grid, dim3(32, 4), 0, st>>>(cases);
   } else {
-    const dim3 grid(batch_x(d->max_lbm_tiles, 1, 1 << 20), d->n_cases);
+    const dim3 grid(batch_grid(d->max_lbm_tiles, d->n_cases, 3, 4), d->n_cases);
     if (d->store_fp16)
       k_batch_lbm_step<true><<<grid, dim3(32, 8), 0, st>>>(cases);
     else
@@ -3164,7 +3157,8 @@ extern "C" int fsi_batch_mask_rebuild(FsiBatchCase* cases, const FsiBatchDims* d
   cudaStream_t st = (cudaStream_t)stream;
   k_batch_ctl<<<d->n_cases, 32, 0, st>>>(cases, kBatchMaskPre);
   if ((rc = launch_check("k_batch_ctl"))) return rc;
-  k_batch_mask_update<<<dim3(batch_x(d->max_cells, 256, 1 << 20), d->n_cases), 256, 0, st>>>(cases);
+  k_batch_mask_update<<<dim3(batch_grid((d->max_cells + 255) / 256, d->n_cases, 8, 4), d->n_cases), 256, 0, st>>>(
+      cases);
   if ((rc = launch_check("k_batch_mask_update"))) return rc;
   const dim3 g2(std::max(1, lbm_sm_count() * 4 / std::max(1, d->n_cases)), d->n_cases);
   if (d->store_fp16)
