@@ -500,6 +500,18 @@ __device__ __forceinline__ void reaction_particle_staged(const float* __restrict
   reaction_from_sums(cp, hs, sum[3], Jp, vol0, scale, r);
 }
 
+// Parts that a sequence cuts its chunks into: twice as many while every part
+// still has a CTA of its own (the substep then takes as long as one part) and a
+// box record, up to max_split (1 where other cases fill the device)
+__device__ __forceinline__ int seq_split(int nbin, int ctas, int records, int max_split) {
+  int split = 1;
+  while (2 * split <= max_split && nbin * split * 2 <= min(ctas, records)) split *= 2;
+  return split;
+}
+
+// CTAs that take part: one per item and half as many to zero old boxes
+__device__ __forceinline__ int seq_ctas_used(int items) { return items + (items >> 1) + 8; }
+
 // one particle's part of the reaction diagnostics
 struct ReactStats {
   int act;              // reaction not zero
@@ -540,12 +552,12 @@ __device__ __forceinline__ ReactStats reaction_stats(const ReactParticle& rp, co
 }
 
 // launch A.s of the sequence for the chunks vb, vb + vg, ... (kSeqT threads,
-// kSeqSmem bytes of dynamic shared memory).  PDL: launched with programmatic
-// stream serialization; what is read before the wait (the chunk table, perm,
-// mass, vol0, fixed) was complete before the launch before the last one, and
-// every launch of the sequence waits for the one before it.
-template <bool REACT, bool PDL>
-__device__ __forceinline__ void mpm_seq_body(const SeqArgs& A, int vb, int vg) {
+// kSeqSmem bytes of dynamic shared memory), launched with programmatic stream
+// serialization: what is read before the wait (the chunk table, perm, mass,
+// vol0, fixed) was complete before the launch before the last one, and every
+// launch of the sequence waits for the one before it.
+template <bool REACT>
+__device__ __forceinline__ void mpm_seq_body(const SeqArgs& A, int vb, int vg, int max_split) {
   constexpr int T = kSeqT, NW = T / 32;
   constexpr int NQ = REACT ? 7 : 4;  // grid values a substep writes
   extern __shared__ float4 seq_smem4[];
@@ -557,13 +569,6 @@ __device__ __forceinline__ void mpm_seq_body(const SeqArgs& A, int vb, int vg) {
   __shared__ int s_cnt[NW];
   __shared__ float s_fmax[NW][2];
   __shared__ double s_dsum[NW][6];
-  if (PDL) {
-    // the launch's arguments into the constant caches while the previous
-    // launch still runs (a first access after the wait costs a trip to L2)
-    const int* const w = reinterpret_cast<const int*>(&A);
-#pragma unroll
-    for (int i = 0; i < (int)(sizeof(SeqArgs) / 4); i += 16) asm volatile("" ::"r"(w[i]));
-  }
   const FsiParticles& pt = A.pt;
   const FsiMpmParams& mp = A.mp;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -575,13 +580,12 @@ __device__ __forceinline__ void mpm_seq_body(const SeqArgs& A, int vb, int vg) {
   const int bg = (s + 2) % 3, bs = s % 3, bz = (s + 1) % 3;
   const int G = A.grid[0].n;
   const int64_t N = (int64_t)G * G * G;
-  // work items: the chunks, each cut into `split` parts where that still gives
-  // every part a CTA of its own (the substep then takes as long as one part)
+  // work items: the chunks, each cut into `split` parts
   const int nbin = A.meta[kMetaChunks];
-  int split = 1;
-  if (PDL)
-    while (split < 4 && nbin * split * 2 <= vg) split *= 2;
+  const int split = seq_split(nbin, vg, (int)(A.box_stride / 6), max_split);
   const int nch = nbin * split;
+  vg = min(vg, seq_ctas_used(nch));
+  if (vb >= vg) return;
   // this thread's particle of the CTA's first item
   int2 ch = make_int2(0, 0);
   int p = 0, pfixed = 0;
@@ -598,10 +602,8 @@ __device__ __forceinline__ void mpm_seq_body(const SeqArgs& A, int vb, int vg) {
     }
   };
   if (vb < nch) load_chunk(vb);
-  if (PDL) {
-    griddep_wait();
-    griddep_launch();
-  }
+  griddep_wait();
+  griddep_launch();
   FsiCouplingStats* const st = REACT ? A.stats + bs : nullptr;
   if (vb == 0 && tid == 0) {
     if (s == 0) {  // the prologue zeroed every buffer
@@ -1000,7 +1002,12 @@ __global__ __launch_bounds__(kSeqT) void k_mpm_seq_prologue(const __grid_constan
 
 template <bool REACT>
 __global__ __launch_bounds__(kSeqT, kSeqOcc) void k_mpm_seq(const __grid_constant__ SeqArgs A) {
-  mpm_seq_body<REACT, true>(A, blockIdx.x, gridDim.x);
+  // the launch's arguments into the constant caches while the previous launch
+  // still runs (a first access after the wait costs a trip to L2)
+  const int* const w = reinterpret_cast<const int*>(&A);
+#pragma unroll
+  for (int i = 0; i < (int)(sizeof(SeqArgs) / 4); i += 16) asm volatile("" ::"r"(w[i]));
+  mpm_seq_body<REACT>(A, blockIdx.x, gridDim.x, 4);
 }
 
 __global__ void k_grid_velocity(FsiGrid g, FsiMpmParams mp, float* __restrict__ out) {
@@ -1213,12 +1220,15 @@ __global__ void k_batch_bin_scatter(const FsiBatchCase* __restrict__ cases) {
     bin_scatter_body(bc.pt.n, bc.bins.key, bc.bins.start, bc.bins.perm, vb, nvb);
 }
 
-// the sequence arguments of a batched case (one thread, into shared memory)
+// the sequence arguments of a batched case, into shared memory by the CTA
+// (read by one thread they were a chain of 60 loads)
 __device__ __forceinline__ void load_batch_seq(const FsiBatchCase& bc, int s, int M, SeqArgs* A) {
-  A->pt = bc.pt;
-#pragma unroll
-  for (int b = 0; b < 3; ++b) A->grid[b] = bc.grid[b];
-  A->mp = bc.mp;
+  const int tid = threadIdx.x, nt = blockDim.x;
+  copy_words(&A->pt, &bc.pt, sizeof(FsiParticles), tid, nt);
+  copy_words(A->grid, bc.grid, 3 * sizeof(FsiGrid), tid, nt);
+  copy_words(&A->mp, &bc.mp, sizeof(FsiMpmParams), tid, nt);
+  copy_words(&A->cp, &bc.cp, sizeof(FsiCouplingParams), tid, nt);
+  if (tid != 0) return;
   A->perm = bc.bins.perm;
   A->chunks = reinterpret_cast<const int2*>(bc.bins.chunk);
   A->meta = bc.bins.meta;
@@ -1227,7 +1237,6 @@ __device__ __forceinline__ void load_batch_seq(const FsiBatchCase& bc, int s, in
   A->L = LatView{bc.lbm.nx, bc.lbm.ny, bc.lbm.nz, bc.lbm.pitch};
   A->hydro = batch_hydro(bc);
   A->phi = bc.lbm.phi;
-  A->cp = bc.cp;
   A->stats = bc.react_stats;
   A->diag = bc.lbm.diag;
   A->s = s;
@@ -1238,18 +1247,30 @@ __global__ __launch_bounds__(kSeqT) void k_batch_mpm_seq_prologue(const FsiBatch
   __shared__ SeqArgs A;
   const FsiBatchCase& bc = cases[blockIdx.y];
   if (!bc.active) return;
-  if (threadIdx.x == 0) load_batch_seq(bc, 0, 1, &A);
+  load_batch_seq(bc, 0, 1, &A);
   __syncthreads();
   seq_prologue_body(A, blockIdx.x, gridDim.x);
 }
 
-__global__ __launch_bounds__(kSeqT, kSeqOcc) void k_batch_mpm_seq(const FsiBatchCase* __restrict__ cases, int s, int M) {
+// Launched with programmatic stream serialization, like k_mpm_seq: the case
+// records and the bins are complete before the prologue starts.
+__global__ __launch_bounds__(kSeqT, kSeqOcc) void k_batch_mpm_seq(const FsiBatchCase* __restrict__ cases, int s, int M,
+                                                                  int max_split) {
   __shared__ SeqArgs A;
   const FsiBatchCase& bc = cases[blockIdx.y];
-  if (!bc.active) return;
-  if (threadIdx.x == 0) load_batch_seq(bc, s, M, &A);
+  if (!bc.active) {
+    if (blockIdx.x == 0) griddep_wait();  // a launch of empty slots must not end before the one ahead of it
+    return;
+  }
+  {
+    // the grid is sized for the largest case: CTAs beyond this case's share leave before the arguments are staged
+    const int nbin = bc.bins.meta[kMetaChunks];
+    const int split = seq_split(nbin, gridDim.x, bc.bins.max_chunks, max_split);
+    if ((int)blockIdx.x >= seq_ctas_used(nbin * split)) return;
+  }
+  load_batch_seq(bc, s, M, &A);
   __syncthreads();
-  mpm_seq_body<true, false>(A, blockIdx.x, gridDim.x);
+  mpm_seq_body<true>(A, blockIdx.x, gridDim.x, max_split);
 }
 
 __global__ __launch_bounds__(kSortT) void k_batch_bin_sort(const FsiBatchCase* __restrict__ cases) {
@@ -1313,9 +1334,13 @@ extern "C" int fsi_batch_mpm_substeps(FsiBatchCase* cases, const FsiBatchDims* d
   const dim3 gc(gx, d->n_cases);
   k_batch_mpm_seq_prologue<<<gc, kSeqT, 0, st>>>(cases);
   if ((rc = launch_check("k_batch_mpm_seq_prologue"))) return rc;
+  // chunks of all cases if each were as large as the largest, against the CTAs the device holds at once
+  const int64_t chunks = (int64_t)nblk(d->max_particles, kChunk) * d->n_cases, room = (int64_t)sm_count() * kSeqOcc;
+  const int max_split = chunks * 4 <= room ? 4 : (chunks * 2 <= room ? 2 : 1);
   for (int i = 0; i <= n_substeps; ++i) {
-    k_batch_mpm_seq<<<gc, kSeqT, kSeqSmem, st>>>(cases, i, n_substeps);
-    if ((rc = launch_check("k_batch_mpm_seq"))) return rc;
+    const cudaError_t lerr = launch_pdl(k_batch_mpm_seq, gc, dim3(kSeqT), kSeqSmem, st, (const FsiBatchCase*)cases, i,
+                                        n_substeps, max_split);
+    if ((rc = cuda_check(lerr, "k_batch_mpm_seq (launch)")) || (rc = launch_check("k_batch_mpm_seq"))) return rc;
   }
   return FSI_OK;
 }
