@@ -420,13 +420,13 @@ int fsi_project(const FsiLbmState* s, const FsiParticles* pt, const FsiCouplingP
  * threshold.  fsi_project's float atomics sum in an unspecified order.
  * Particles are sorted by B-spline base cell over the bounding box of the
  * base cells; each cell then gathers its contributors (at most 27 base-cell
- * lists), ranks them by particle index and sums them in rank order. */
+ * lists), sorts them by particle index and sums them in that order. */
 typedef struct FsiProjectScratch {
   int32_t key_capacity;       /* >= (nx + 2) * (ny + 2) * (nz + 2) */
   int32_t particle_capacity;  /* >= the particle count */
   int32_t* count;             /* [key_capacity + 1], zero before the first call; kept zero after each call */
   int32_t* start;             /* [key_capacity + 1] */
-  int32_t* list;              /* [particle_capacity] particle ids by base cell, ascending within a cell */
+  int32_t* list;              /* [particle_capacity] particle ids by base cell */
   int32_t* key;               /* [particle_capacity] */
   int32_t* box;               /* [8] base-cell bounding box of the last call */
 } FsiProjectScratch;

@@ -1,4 +1,11 @@
-"""The float-atomic projection (fsi_project, the batched form's) at the edges of
+"""Edges of both projections' launches.
+
+The ordered projection (fsi_project_ordered) against the oracle, bit for bit:
+cells whose number of contributors lies at the sizes where the register sort
+changes and where the ids are taken in several passes, and bounding boxes whose
+keys end at, before and after the blocks of the scan.
+
+The float-atomic projection (fsi_project, the batched form's) at the edges of
 its warp-wide runs: one particle, partly filled warps, particles in memory order
 and shuffled, one crowded cell, stencils that leave the lattice.  Compared with
 the serial order's sums (fsi_project_ordered): a cell adds at most K terms in
@@ -56,3 +63,46 @@ def test_unordered_projection_matches_ordered(kind):
     got = proj.get_stats()
     assert got["active_cell_count"] == want["active_cell_count"]
     np.testing.assert_allclose(got["projected_mass"], want["projected_mass"], rtol=rel)
+
+
+def _ordered_cloud(kind, rng):
+    if kind == "counts":  # one base cell each, far apart
+        counts = (1, 2, 31, 32, 33, 64, 65, 127, 128, 129, 256, 257, 511, 512, 513, 1024, 1025, 1600)
+        cells = [(3 + 6 * (i % 3), 3 + 6 * (i // 3 % 3), 3 + 9 * (i // 9)) for i in range(len(counts))]
+        x = np.concatenate([np.array(c) + rng.uniform(0.55, 1.45, (m, 3)) for c, m in zip(cells, counts)])
+        return rng.permutation(x)
+    # keys = 15 * 15 * 18 = 4050, 16 * 16 * 16 = 4096, 17 * 15 * 17 = 4335, 24 ** 3 = 13824
+    ext = np.array({"keys_4050": (15, 15, 18), "keys_4096": (16, 16, 16), "keys_4335": (17, 15, 17),
+                    "keys_13824": (24, 24, 24)}[kind])
+    lo = np.minimum(2, N - ext)
+    x = lo + 0.5 + np.floor(rng.uniform(0, 1, (700, 3)) * ext) + rng.uniform(0.05, 0.95, (700, 3))
+    return np.concatenate([x, [lo + 0.7], [lo + ext - 0.3]])
+
+
+@pytest.mark.parametrize("kind", ["counts", "keys_4050", "keys_4096", "keys_4335", "keys_13824"])
+def test_ordered_projection_launch_edges(kind):
+    from mpm_lbm_b200.config import LBMConfig, MPMConfig, UnifiedSimConfig
+    from mpm_lbm_b200.coupling import MPMToLBMProjector3D
+    from mpm_lbm_b200.lbm import LBMFluid3D
+    from mpm_lbm_b200.mpm import MPMSolid3D
+    from oracle import oracle as orc
+
+    rng = np.random.default_rng(5)
+    x = (_ordered_cloud(kind, rng) / N).astype(np.float32)
+    n = len(x)
+    vol = np.full(n, (1.0 / N) ** 3 / 8, np.float32)
+    mass = vol * np.float32(1.2)
+    v = rng.standard_normal((n, 3)).astype(np.float32)
+    sim = UnifiedSimConfig(n_grid=N, mpm_dt=1e-4, lbm_dt_phys_override_s=1.0e-3)
+    lbm = LBMFluid3D(LBMConfig(nx=N, ny=N, nz=N))
+    solid = MPMSolid3D(MPMConfig(n_grid=N, dx=1.0 / N, dt=1e-4), n)
+    solid.init_from_numpy(x, vol, mass, v_np=v)
+    ol, om = orc.OracleLBM(N, N, N), orc.OracleMPM(N, 1.0 / N, 1e-4, n)
+    om.x[...], om.v[...], om.Jp[...], om.vol0[...], om.mass[...] = x, v, 1.0, vol, mass
+    orc.OracleCoupling(N, sim.dx_norm, sim.lbm_dt_phys).project(om, ol)
+    proj = MPMToLBMProjector3D(sim)
+    for _ in range(2):  # the second call finds the scratch as the first one left it
+        proj.project(solid, lbm)
+        np.testing.assert_array_equal(lbm.solid_phi.to_numpy(), ol.solid_phi)
+        np.testing.assert_array_equal(lbm.solid_mass.to_numpy(), ol.solid_mass)
+        np.testing.assert_array_equal(lbm.solid_vel.to_numpy(), ol.solid_vel)
