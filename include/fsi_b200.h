@@ -451,6 +451,10 @@ int fsi_mpm_grid_update(const FsiGrid* g, const FsiMpmParams* mp, void* stream);
  * F update, damping / z-lock controls, fixed-base reset. */
 int fsi_mpm_g2p(const FsiParticles* pt, const FsiGrid* g, const FsiMpmParams* mp, void* stream);
 
+/* MPMSolid3D.substep (mpm/solid.py:212-315): the grid (with f_ext) cleared, then
+ * the three phases above. */
+int fsi_mpm_substep(const FsiParticles* pt, const FsiGrid* g, const FsiMpmParams* mp, void* stream);
+
 /* ---- binned MPM substeps ------------------------------------------------
  * The same substep as clear -> p2g -> reaction -> grid_update -> g2p above
  * (one call of MPMSolid3D.substep plus the coupler's reaction transfer, as

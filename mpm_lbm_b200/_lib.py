@@ -196,6 +196,7 @@ SIGNATURES = {
     "fsi_mpm_p2g": [_P(FsiParticles), _P(FsiGrid), _P(FsiMpmParams), c_p],
     "fsi_mpm_grid_update": [_P(FsiGrid), _P(FsiMpmParams), c_p],
     "fsi_mpm_g2p": [_P(FsiParticles), _P(FsiGrid), _P(FsiMpmParams), c_p],
+    "fsi_mpm_substep": [_P(FsiParticles), _P(FsiGrid), _P(FsiMpmParams), c_p],
     "fsi_mpm_bins_layout": [c_i32, c_i32, _P(c_i32), _P(c_i32)],
     "fsi_mpm_bin": [_P(FsiParticles), _P(FsiGrid), _P(FsiMpmParams), _P(FsiMpmBins), c_p],
     "fsi_mpm_substeps_binned": [_P(FsiParticles), _P(FsiGrid), _P(FsiMpmBins), _P(FsiMpmParams), c_i32,

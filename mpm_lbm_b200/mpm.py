@@ -231,10 +231,9 @@ class MPMSolid3D:
              self._stream())
 
     def substep(self):
-        self.clear_grid()
-        self.p2g()
-        self.grid_update()
-        self.g2p()
+        self._one_phase_grid()
+        call("fsi_mpm_substep", ctypes.byref(self.particles), ctypes.byref(self.grid), ctypes.byref(self.params),
+             self._stream())
 
     # ---- binned substep -------------------------------------------------
     def _ensure_binned(self):
