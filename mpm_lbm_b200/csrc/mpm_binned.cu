@@ -49,7 +49,7 @@ __device__ __forceinline__ int particle_bin(const float X[3], float inv_dx, int 
 }
 
 __device__ __forceinline__ void bin_count_body(const FsiParticles& pt, float inv_dx, int G, int nb,
-                                               int32_t* __restrict__ key, int32_t* __restrict__ count, int vb, int vg) {
+                                               int32_t* key, int32_t* count, int vb, int vg) {
   const int p = vb * blockDim.x + threadIdx.x;
   if (p >= pt.n) return;
   const int n = pt.n;
@@ -59,8 +59,9 @@ __device__ __forceinline__ void bin_count_body(const FsiParticles& pt, float inv
   atomicAdd(count + k, 1);
 }
 
-__global__ void k_bin_count(FsiParticles pt, float inv_dx, int G, int nb, int32_t* __restrict__ key,
-                            int32_t* __restrict__ count) {
+__global__ void k_bin_count(FsiParticles pt, float inv_dx, int G, int nb, int32_t* key, int32_t* count) {
+  griddep_wait();
+  griddep_launch();
   bin_count_body(pt, inv_dx, G, nb, key, count, blockIdx.x, gridDim.x);
 }
 
@@ -83,8 +84,8 @@ __device__ __forceinline__ int4 ld_bins4(const int32_t* p, int b, int b1) {
 
 __device__ __forceinline__ int chunks_of(int c) { return (c + kChunk - 1) / kChunk; }
 
-__device__ __forceinline__ void bin_scan_body(int nbins, int32_t* __restrict__ count, int32_t* __restrict__ start,
-                                              int2* __restrict__ chunk, int32_t* __restrict__ meta) {
+__device__ __forceinline__ void bin_scan_body(int nbins, int32_t* count, int32_t* start, int2* chunk,
+                                              int32_t* meta) {
   __shared__ int s_p[32], s_c[32];
   const int T = blockDim.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int per = ((nbins + T - 1) / T + 3) & ~3;
@@ -160,22 +161,23 @@ __device__ __forceinline__ void bin_scan_body(int nbins, int32_t* __restrict__ c
   if (tid == T - 1) meta[0] = co;
 }
 
-__global__ __launch_bounds__(1024) void k_bin_scan(int nbins, int32_t* __restrict__ count,
-                                                   int32_t* __restrict__ start, int2* __restrict__ chunk,
-                                                   int32_t* __restrict__ meta) {
+__global__ __launch_bounds__(1024) void k_bin_scan(int nbins, int32_t* count, int32_t* start, int2* chunk,
+                                                   int32_t* meta) {
+  griddep_wait();
+  griddep_launch();
   bin_scan_body(nbins, count, start, chunk, meta);
 }
 
-__device__ __forceinline__ void bin_scatter_body(int n, const int32_t* __restrict__ key,
-                                                 int32_t* __restrict__ cursor, int32_t* __restrict__ perm, int vb,
-                                                 int vg) {
+__device__ __forceinline__ void bin_scatter_body(int n, const int32_t* key, int32_t* cursor, int32_t* perm,
+                                                 int vb, int vg) {
   const int p = vb * blockDim.x + threadIdx.x;
   if (p >= n) return;
   perm[atomicAdd(cursor + key[p], 1)] = p;
 }
 
-__global__ void k_bin_scatter(int n, const int32_t* __restrict__ key, int32_t* __restrict__ cursor,
-                              int32_t* __restrict__ perm) {
+__global__ void k_bin_scatter(int n, const int32_t* key, int32_t* cursor, int32_t* perm) {
+  griddep_wait();
+  griddep_launch();
   bin_scatter_body(n, key, cursor, perm, blockIdx.x, gridDim.x);
 }
 
@@ -198,8 +200,8 @@ __device__ __forceinline__ int local_base_cell(const FsiParticles& pt, int p, fl
 }
 
 __device__ __forceinline__ void bin_sort_body(const FsiParticles& pt, float inv_dx, int G, int nbins,
-                                              const int32_t* __restrict__ end, int32_t* __restrict__ perm,
-                                              int32_t* __restrict__ tmp, int vb, int vg) {
+                                              const int32_t* end, int32_t* perm,
+                                              int32_t* tmp, int vb, int vg) {
   __shared__ int cnt[kBinCells];
   __shared__ int wsum[kSortT / 32];
   const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
@@ -246,8 +248,10 @@ __device__ __forceinline__ void bin_sort_body(const FsiParticles& pt, float inv_
 }
 
 __global__ __launch_bounds__(kSortT) void k_bin_sort(FsiParticles pt, float inv_dx, int G, int nbins,
-                                                      const int32_t* __restrict__ end, int32_t* __restrict__ perm,
-                                                      int32_t* __restrict__ tmp) {
+                                                      const int32_t* end, int32_t* perm,
+                                                      int32_t* tmp) {
+  griddep_wait();
+  griddep_launch();
   bin_sort_body(pt, inv_dx, G, nbins, end, perm, tmp, blockIdx.x, gridDim.x);
 }
 
@@ -1110,17 +1114,29 @@ extern "C" int fsi_mpm_bin(const FsiParticles* pt, const FsiGrid* g, const FsiMp
   if ((rc = check_bins(bins, pt->n, g->n))) return rc;
   cudaStream_t st = (cudaStream_t)stream;
   const int nb = (g->n + kEdge - 1) / kEdge;
-  k_bin_count<<<nblk(pt->n, 256), 256, 0, st>>>(*pt, mp->inv_dx, g->n, nb, bins->key, bins->count);
-  if ((rc = launch_check("k_bin_count"))) return rc;
-  k_bin_scan<<<1, 1024, 0, st>>>(bins->n_bins, bins->count, bins->start, reinterpret_cast<int2*>(bins->chunk),
-                                 bins->meta);
-  if ((rc = launch_check("k_bin_scan"))) return rc;
-  k_bin_scatter<<<nblk(pt->n, 256), 256, 0, st>>>(pt->n, bins->key, bins->start, bins->perm);
-  if ((rc = launch_check("k_bin_scatter"))) return rc;
+  // four launches of 3-5 us for a few thousand particles, each started while the
+  // one before drains (none of their pointers is __restrict__: no load may move
+  // above griddep_wait()); with the mask rebuild's launches likewise, a 32^3 FSI
+  // step of 10 substeps 243 -> 226 us
+  auto launched = [&](cudaError_t e, const char* what) {
+    const int r = cuda_check(e, what);
+    return r ? r : launch_check(what);
+  };
+  const dim3 pb(nblk(pt->n, 256)), t(256);
+  if ((rc = launched(launch_pdl(k_bin_count, pb, t, 0, st, *pt, mp->inv_dx, g->n, nb, bins->key, bins->count),
+                     "k_bin_count")))
+    return rc;
+  if ((rc = launched(launch_pdl(k_bin_scan, dim3(1), dim3(1024), 0, st, bins->n_bins, bins->count, bins->start,
+                                reinterpret_cast<int2*>(bins->chunk), bins->meta),
+                     "k_bin_scan")))
+    return rc;
+  if ((rc = launched(launch_pdl(k_bin_scatter, pb, t, 0, st, pt->n, bins->key, bins->start, bins->perm),
+                     "k_bin_scatter")))
+    return rc;
   // the bin keys are no longer needed: key[] is the sort's scratch
-  k_bin_sort<<<(unsigned)std::min(bins->n_bins, sm_count() * 8), kSortT, 0, st>>>(
-      *pt, mp->inv_dx, g->n, bins->n_bins, bins->start, bins->perm, bins->key);
-  return launch_check("k_bin_sort");
+  return launched(launch_pdl(k_bin_sort, dim3((unsigned)std::min(bins->n_bins, sm_count() * 8)), dim3(kSortT), 0, st,
+                             *pt, mp->inv_dx, g->n, bins->n_bins, bins->start, bins->perm, bins->key),
+                  "k_bin_sort");
 }
 
 extern "C" int fsi_mpm_substeps_binned(const FsiParticles* pt, const FsiGrid grid[3], const FsiMpmBins* bins,

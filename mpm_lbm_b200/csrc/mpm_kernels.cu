@@ -297,8 +297,8 @@ __device__ __forceinline__ int ordered_key(const OrdBox& B, const int b[3]) {
   return ((b[2] - B.lo[2]) * B.ext[1] + (b[1] - B.lo[1])) * B.ext[0] + (b[0] - B.lo[0]);
 }
 
-__global__ void k_po_count(LatView L, FsiParticles pt, float inv_dx, const int32_t* box,
-                           int32_t* key, int32_t* count) {
+__global__ void k_po_count(LatView L, FsiParticles pt, float inv_dx, const int32_t* box, int32_t* key,
+                           int32_t* count) {
   griddep_wait();
   griddep_launch();
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
