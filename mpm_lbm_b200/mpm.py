@@ -126,7 +126,11 @@ class MPMSolid3D:
         self._binned_clean = True  # the buffers are zero outside the recorded boxes
         self._binned_mode = "seq"
         self._since_bin = 0
-        self.rebin_interval = 64  # binned substeps between automatic re-binnings
+        # binned substeps between automatic re-binnings.  As particles cross cells a chunk's node box grows (to three
+        # times its nodes within some ten substeps of a moving body) and its scatter with it.  Four substeps, moving /
+        # at rest, every 64 -> every 8: 222,000 particles 403 -> 360 / 287 -> 305 us, 500,000 841 -> 726 / 617 -> 602,
+        # 1,000,000 1,827 -> 1,529 / 1,098 -> 1,080; 98,000 209 -> 216 / 150 -> 186.
+        self.rebin_interval = 8 if self.n_particles >= 3 << 17 else 64
 
     def _stream(self):
         return stream_handle()
