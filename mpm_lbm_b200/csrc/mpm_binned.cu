@@ -373,7 +373,7 @@ enum { kQmass = 36, kQkey = 40, kQn = 44 };
 // One substep, before (two threads per particle, 8 warps, tile with
 // shared-memory atomics) and now, with the binning's share: 19.7 -> 14.9 us
 // (4,096 particles), 24.4 -> 21.7 us (24,576), 124 -> 87 us (196,608); the
-// 16-case batch's 11 launches 1,312 -> 700 us.  Three threads per particle (12
+// 16-case batch's 11 launches 1,312 -> 630 us.  Three threads per particle (12
 // warps, one axis each) took 13-21 us at the small sizes but 116 us at 196,608
 // particles and no less than before in a batch.
 
