@@ -2779,8 +2779,9 @@ extern "C" int fsi_lbm_substeps(const FsiLbmState* s, const FsiLbmParams* p, con
   if (rc) return rc;
   if (!ctl) return invalid("null step control");
   if (n < 0) return invalid("n must be >= 0");
-  if (!(ctl->mode & FSI_MODE_MOVING_BB) || (ctl->mode & (FSI_MODE_DIRSTATS | FSI_MODE_PENALTY)))
-    return invalid("fsi_lbm_substeps takes moving-boundary substeps without per-direction reductions or penalty force");
+  if (!(ctl->mode & FSI_MODE_MOVING_BB) || (ctl->mode & FSI_MODE_DIRSTATS))
+    return invalid("fsi_lbm_substeps takes moving-boundary substeps without per-direction reductions");
+  if (ctl->mode & FSI_MODE_PENALTY) return invalid("penalty steps use static bounce-back (fluid.py:2099-2103)");
   FsiStepCtl k = *ctl;
   for (int32_t i = 0; i < n; ++i) {
     if ((rc = fsi_lbm_substep(s, p, &k, stream))) return rc;

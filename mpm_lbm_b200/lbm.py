@@ -440,6 +440,8 @@ class LBMFluid3D:
         if self.tau_f is None:
             raise RuntimeError("init_simulation() must run before stepping")
         mode = FSI_MODE_MOVING_BB | (FSI_MODE_SUBCYCLED if self._accumulating else 0)
+        if self._penalty is not None:  # refused, as by step_moving_bounceback()
+            mode |= FSI_MODE_PENALTY
         self._sync_params()
         ctl = self._ctl(mode)
         call("fsi_lbm_substeps", ctypes.byref(self.state), ctypes.byref(self.params), ctypes.byref(ctl), int(n),
@@ -450,7 +452,6 @@ class LBMFluid3D:
         self.bc_pending = bool(self.bc_x_left or self.bc_x_right)
         self.steps += n
         self._version += n
-        self._penalty = None
         self._hydro_src = self.last_pp
         self._fused_accumulation = self._accumulating
         if self._accumulating:
