@@ -293,13 +293,12 @@ __device__ __forceinline__ float grid_node_component(float P, float im, float f,
 // G2P sums of a particle whose stencil leaves the grid, or whose chunk's node
 // box does not fit the shared-memory stage (bins gone stale): a rolled loop
 // over the nodes inside the grid, from the stage when stg is non-null, from
-// the grid otherwise.
+// the grid otherwise, a node's seven values requested together.
 __device__ __noinline__ void g2p_slow(const float* stg, int nv, const Box& bx, const FsiGrid& g, const FsiMpmParams& mp,
                                       const BSpline& b, float s4, float v[3], float nC[9]) {
   const int G = g.n;
   const int64_t N = (int64_t)G * G * G;
-  for (int a = 0; a < 3; ++a) v[a] = 0.f;
-  for (int a = 0; a < 9; ++a) nC[a] = 0.f;
+  float sv[3] = {0.f, 0.f, 0.f}, sC[9] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll 1
   for (int o = 0; o < 27; ++o) {
     const int ox = o / 9, oy = (o / 3) % 3, oz = o % 3;
@@ -309,17 +308,33 @@ __device__ __noinline__ void g2p_slow(const float* stg, int nv, const Box& bx, c
     const float d[3] = {((float)ox - b.fx[0]) * mp.dx, ((float)oy - b.fx[1]) * mp.dx, ((float)oz - b.fx[2]) * mp.dx};
     const int li = ((id[2] - bx.lo[2]) * bx.ext[1] + (id[1] - bx.lo[1])) * bx.ext[0] + (id[0] - bx.lo[0]);
     const int64_t node = ((int64_t)id[2] * G + id[1]) * G + id[0];
-    const float m = stg ? 0.f : g.m[node], im = m > 0.f ? __frcp_rn(m) : 0.f;
+    float gv[3];
+    if (stg) {
+#pragma unroll
+      for (int a = 0; a < 3; ++a) gv[a] = stg[a * nv + li];
+    } else {
+      const float m = g.m[node];
+      const float f[3] = {g.f_ext[node], g.f_ext[N + node], g.f_ext[2 * N + node]};  // all in flight together
+#pragma unroll
+      for (int a = 0; a < 3; ++a) gv[a] = g.v[a * N + node];
+      if (m > 0.f) {
+        const float im = __frcp_rn(m);
+#pragma unroll
+        for (int a = 0; a < 3; ++a) gv[a] = grid_node_component(gv[a], im, f[a], mp.gravity[a], id[a], G, mp);
+      }
+    }
+#pragma unroll
     for (int a = 0; a < 3; ++a) {
-      const float gv = stg ? stg[a * nv + li]
-                           : (m > 0.f ? grid_node_component(g.v[a * N + node], im, g.f_ext[a * N + node],
-                                                            mp.gravity[a], id[a], G, mp)
-                                      : g.v[a * N + node]);
-      const float wg = w * gv;
-      v[a] += wg;
-      for (int k = 0; k < 3; ++k) nC[a * 3 + k] += wg * d[k] * s4;
+      const float wg = w * gv[a];
+      sv[a] += wg;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) sC[a * 3 + k] += wg * d[k] * s4;
     }
   }
+#pragma unroll
+  for (int a = 0; a < 3; ++a) v[a] = sv[a];
+#pragma unroll
+  for (int a = 0; a < 9; ++a) nC[a] = sC[a];
 }
 
 // P2G payload of a particle (shared memory), one record of kQn floats per
