@@ -27,12 +27,10 @@ namespace {
 
 constexpr int kChunk = FSI_BIN_CHUNK;  // particles per chunk
 constexpr int kEdge = FSI_BIN_EDGE;
-// nodes staged per CTA: the stencils of a chunk of one bin span at most
-// (8 + 2)^3 = 1000 nodes; the rest absorbs a node of drift since the last
-// binning (an 11^3 box).  Two regions of shared memory: the scatter tile (7
-// floats per node, 37 KB) and the stage of the gather's node velocities and of
-// the reaction's lattice box (4 floats per node), so that the tile can be
-// zeroed while the payload is built.
+// nodes of a chunk's box that are staged in shared memory: the stencils of a
+// chunk of one bin span at most (8 + 2)^3 = 1000 nodes; the rest absorbs a node
+// of drift since the last binning (an 11^3 box).  A wider box is read from and
+// added to the grid directly.
 constexpr int kTileCap = 1331;
 
 __device__ __forceinline__ int clampi(int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); }
@@ -347,7 +345,8 @@ __device__ __noinline__ void g2p_slow(const float* stg, int nv, const Box& bx, c
 //   [4 (3 a + o)] share0 share1 share2 weight   (a = 0: m v is in the share)
 //   [36] mass pf0 pf1 pf2                      [40] key base0 base1 base2
 // key: the index of the base node in the chunk's box (int bits), -1 when the
-// stencil leaves the grid or the chunk's box is too large; base as int bits.
+// stencil leaves the grid or the chunk's box is too large; base as int bits,
+// modulo 3 where one or two tiles fit the box and the key is not -1.
 // A record of 44 floats keeps the 128-bit stores of 8 consecutive particles
 // on distinct banks.
 enum { kQmass = 36, kQkey = 40, kQn = 44 };
@@ -355,19 +354,16 @@ enum { kQmass = 36, kQkey = 40, kQn = 44 };
 // ---- fused substep sequence --------------------------------------------------
 // M substeps in M + 1 launches (after a prologue).  Launch s, for each chunk of
 // its CTA: the gather of substep s - 1 (G2P from grid buffer (s - 1) % 3, the
-// new particle state written to the particle fields and kept in shared
-// memory), then the P2G payload of substep s from that state and its scatter
-// into buffer s % 3.  A chunk's particles belong to one CTA for the launch, so
+// new particle state written to the particle fields and kept in registers),
+// then the P2G payload of substep s from that state and its scatter into
+// buffer s % 3.  A chunk's particles belong to one CTA for the launch, so
 // gather, payload and scatter of a chunk follow each other without any
 // grid-wide synchronisation; the launch boundary is the one grid-wide step
 // (every scatter of substep s is complete before any gather of it).  The
 // launch also zeroes the boxes substep s - 2 recorded in buffer (s + 1) % 3,
 // whose last reader (the gather of substep s - 2) ran in the launch before:
 // three buffers, so that no launch zeroes a buffer that another CTA of the
-// same launch still reads or writes.  The arithmetic is the one of the
-// three-kernel substep above (p2g_particle, reaction_particle, g2p_node and
-// g2p_finish on the same values).
-
+// same launch still reads or writes.
 //
 // A CTA has one thread per particle of the chunk (four warps), which keeps the
 // particle's state in registers from the gather to the payload; the scatter
@@ -391,6 +387,10 @@ enum { kQmass = 36, kQkey = 40, kQn = 44 };
 // 16-case batch's 11 launches 1,312 -> 630 us.  Three threads per particle (12
 // warps, one axis each) took 13-21 us at the small sizes but 116 us at 196,608
 // particles and no less than before in a batch.
+// Particles at random positions, with the reaction, at 8 / 2 / 0.5 / 0.125 per
+// cell, that earlier form and this one: 24,576 particles 23 / 24 / 28 / 58 us and
+// 18 / 21 / 25 / 36 us; 196,608: 105 / 129 / 183 / 359 us and
+// 70 / 93 / 144 / 218 us.
 
 // bins->meta: [0] chunks, [1 + b] records in box[b], [4] chunks scattered
 // without a tile, [5 + b] buffer b holds recorded boxes not yet zeroed
@@ -398,11 +398,15 @@ enum { kMetaChunks = 0, kMetaRec = 1, kMetaOverflow = 4, kMetaDirty = 5 };
 constexpr int kSeqT = kChunk;
 constexpr int kSeqOcc = 4;          // resident CTAs per SM (by registers and by shared memory)
 // one region for the staged node velocities (G2P, 3 per node), the reaction's
-// lattice box (4 per cell) and the scatter tiles (7 per node and copy): each is
-// written after the last read of the one before it.  Four copies of the tile
-// fit for boxes of up to 243 nodes (a compact chunk of 128 particles at 8 per
-// cell has 120-220), two for 486, one for 972.
-constexpr int kStageFloats = 6816;
+// lattice box (4 per cell) and the scatter tiles (7 values per node and copy
+// with the reaction, 4 without): each is written after the last read of the one
+// before it.  Four copies of the tile fit boxes of up to 292 nodes with the
+// reaction (512 without), two 585 (1,024), one 1,170 (all that are staged).  A
+// compact chunk of 128 particles at 8 per cell has 120-220 nodes, at 2 per cell
+// 270-440, at one per two cells 440-770.  The size is what four CTAs of an SM
+// can have; a sixth less (243, 486 and 973 nodes) was up to 6 % slower at 0.5 to
+// 4 particles per cell and no faster anywhere.
+constexpr int kStageFloats = 8192;
 static_assert(kStageFloats >= 4 * kTileCap && kStageFloats % 4 == 0, "stage holds the lattice box");
 constexpr size_t kSeqSmem = sizeof(float) * (kStageFloats + kQn * kChunk);
 
@@ -530,6 +534,133 @@ __device__ __forceinline__ int seq_split(int nbin, int ctas, int records, int ma
 
 // CTAs that take part: one per item and half as many to zero old boxes
 __device__ __forceinline__ int seq_ctas_used(int items) { return items + (items >> 1) + 8; }
+
+// Adds the momentum components a0 .. a0 + NM - 1 and the values f0 .. f0 + NF - 1 of (mass, reaction) of the payload
+// records [first, last) to a tile of nv nodes and box extents e0, e0 x e1.  Lane l takes the nodes of one class of
+// indices modulo 3, of which every stencil holds one: no two lanes meet in a node, so four particles go through
+// together, the sums handed on in registers where they share a node (two at a time were 1-2 % faster where the SMs are
+// full, 10-20 % slower where a chunk has one to itself).
+template <int NM, int NF>
+__device__ __forceinline__ void scatter_values(const float* sp, int first, int last, int a0, int f0, float* tile, int nv,
+                                               int e0, int e01, const FsiGrid& g) {
+  constexpr int NV = NM + NF, U = 4;
+  const int lane = threadIdx.x & 31, G = g.n;
+  const int rx = lane % 3, ry = (lane / 3) % 3, rz = min(lane / 9, 2);  // lanes 27-31 are not used
+  struct Rec {
+    int at;  // node in the box
+    float w, val[NV];
+  };
+  auto read = [&](const float* r, int ox, int oy, int oz, int key) {
+    const float *const x = r + 4 * ox, *const y = r + 12 + 4 * oy, *const z = r + 24 + 4 * oz;
+    Rec c;
+    c.at = key + oz * e01 + oy * e0 + ox;
+    c.w = x[3] * y[3] * z[3];
+#pragma unroll
+    for (int i = 0; i < NM; ++i) c.val[i] = x[a0 + i] + y[a0 + i] + z[a0 + i];
+#pragma unroll
+    for (int i = 0; i < NF; ++i) c.val[NM + i] = r[kQmass + f0 + i];
+    return c;
+  };
+  auto offset = [](int cls, int base) { return cls - base + (cls < base ? 3 : 0); };
+  auto value = [&](int i) { return tile + (i < NM ? a0 + i : 3 + f0 + i - NM) * nv; };
+  int lp = first;
+  while (lp < last) {
+    int4 head[U];
+    int low = 0;
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      head[k] = *reinterpret_cast<const int4*>(sp + min(lp + k, last - 1) * kQn + kQkey);
+      low = min(low, head[k].x);
+    }
+    if (low >= 0 && lp + U <= last) {
+      Rec c[U];
+      float t[U][NV];
+#pragma unroll
+      for (int k = 0; k < U; ++k)
+        c[k] = read(sp + (lp + k) * kQn, offset(rx, head[k].y), offset(ry, head[k].z), offset(rz, head[k].w), head[k].x);
+#pragma unroll
+      for (int k = 0; k < U; ++k)
+#pragma unroll
+        for (int i = 0; i < NV; ++i) t[k][i] = value(i)[c[k].at];
+#pragma unroll
+      for (int k = 0; k < U; ++k) {
+#pragma unroll
+        for (int j = 0; j < k; ++j) {
+          const bool same = c[j].at == c[k].at;
+#pragma unroll
+          for (int i = 0; i < NV; ++i) t[k][i] = same ? t[j][i] : t[k][i];
+        }
+#pragma unroll
+        for (int i = 0; i < NV; ++i) t[k][i] += c[k].w * c[k].val[i];
+      }
+      if (lane < 27) {
+#pragma unroll
+        for (int k = 0; k < U; ++k)
+#pragma unroll
+          for (int i = 0; i < NV; ++i) value(i)[c[k].at] = t[k][i];
+      }
+      lp += U;
+      continue;
+    }
+    const float* const r = sp + lp * kQn;
+    const int4 h = head[0];
+    if (h.x >= 0) {
+      const Rec c = read(r, offset(rx, h.y), offset(ry, h.z), offset(rz, h.w), h.x);
+      if (lane < 27) {
+#pragma unroll
+        for (int i = 0; i < NV; ++i) value(i)[c.at] += c.w * c.val[i];
+      }
+    } else {
+      // a stencil that leaves the grid: to the grid
+      const Rec c = read(r, rx, ry, rz, 0);
+      const int I = h.y + rx, J = h.z + ry, K = h.w + rz;
+      if (lane < 27 && I >= 0 && I < G && J >= 0 && J < G && K >= 0 && K < G) {
+        const int64_t N = (int64_t)G * G * G, node = ((int64_t)K * G + J) * G + I;
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+          const int f = f0 + i - NM;  // of (mass, reaction)
+          float* const dst = i < NM ? g.v + (a0 + i) * N : (f == 0 ? g.m : g.f_ext + (f - 1) * N);
+          const float x = c.w * c.val[i];
+          if (x != 0.f) atomicAdd(dst + node, x);
+        }
+      }
+    }
+    ++lp;
+  }
+}
+
+// Boxes that only one or two tiles fit: the warps that share a tile divide the grid values between them, so that each
+// adds its values of all the tile's particles, with no turns and no atomics.  Such boxes hold two particles per cell or
+// fewer (sparse clouds), and nearly every particle is a run of its own there.
+template <bool REACT>
+__device__ __forceinline__ void scatter_shared_tiles(const float* sp, int count, int copies, float* stg, int stride,
+                                                     int nv, int e0, int e01, const FsiGrid& g) {
+  constexpr int NW = kSeqT / 32;
+  const int wid = threadIdx.x >> 5;
+  for (int i = threadIdx.x; i < copies * stride / 4; i += kSeqT)
+    reinterpret_cast<float4*>(stg)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  __syncthreads();
+  const int group = NW / copies, c = wid / group, m = wid % group;  // warps per tile, this one's tile and part
+  const int first = c * count / copies, last = (c + 1) * count / copies;
+  float* const tile = stg + c * stride;
+  if (copies == 2) {
+    if (REACT) {
+      if (m == 0)
+        scatter_values<3, 1>(sp, first, last, 0, 0, tile, nv, e0, e01, g);
+      else
+        scatter_values<0, 3>(sp, first, last, 0, 1, tile, nv, e0, e01, g);
+    } else {
+      if (m == 0)
+        scatter_values<2, 0>(sp, first, last, 0, 0, tile, nv, e0, e01, g);
+      else
+        scatter_values<1, 1>(sp, first, last, 2, 0, tile, nv, e0, e01, g);
+    }
+  } else if (m < 3) {
+    scatter_values<1, REACT ? 1 : 0>(sp, first, last, m, 1 + m, tile, nv, e0, e01, g);
+  } else {
+    scatter_values<0, 1>(sp, first, last, 0, 0, tile, nv, e0, e01, g);
+  }
+}
 
 // one particle's part of the reaction diagnostics
 struct ReactStats {
@@ -859,7 +990,10 @@ __device__ __forceinline__ void mpm_seq_body(const SeqArgs& A, int vb, int vg, i
         if (do_stats) st_add = reaction_stats(rp, b, G);
       }
       *reinterpret_cast<float4*>(rq + kQmass) = make_float4(pmass, pf[0], pf[1], pf[2]);
-      *reinterpret_cast<int4*>(rq + kQkey) = make_int4(copies && inside ? li : -1, b.base[0], b.base[1], b.base[2]);
+      const bool to_tile = copies && inside, mod3 = to_tile && copies < 4;
+      *reinterpret_cast<int4*>(rq + kQkey) =
+          make_int4(to_tile ? li : -1, mod3 ? b.base[0] % 3 : b.base[0], mod3 ? b.base[1] % 3 : b.base[1],
+                    mod3 ? b.base[2] % 3 : b.base[2]);
     }
     if (do_stats) {
       // the warp's part of the diagnostics reductions (penalty.py:202-240, moving_boundary.py:312-374)
@@ -896,8 +1030,13 @@ __device__ __forceinline__ void mpm_seq_body(const SeqArgs& A, int vb, int vg, i
     // of some 100 cycles).  Particles are sorted by base node within the chunk
     // (fsi_mpm_bin), so they come in runs of one base node.
     // (1) Each warp sums its runs, one particle at a time, lane o on stencil
-    // node o (lanes 27-31 are not used), and adds a run's 27 x 7 sums to its own copy of the tile.  With
-    // fewer copies than warps the warps take turns.
+    // node o (lanes 27-31 are not used), and adds a run's 27 x 7 sums to its
+    // own copy of the tile, or straight to the grid where no tile fits (each
+    // particle of such a box has most of its nodes to itself).  Where one or
+    // two copies fit, the warps take turns on them if the runs are long, and
+    // divide the values between them if the runs are short: from 2.5 particles a
+    // run on the turns need fewer instructions (98,304 particles at 3 per cell
+    // 55.5 against 58.2 us, at 2 per cell 67.2 against 62.2 us).
     const FsiGrid g = grid_of(A, bs);
     float* const dst[7] = {g.v, g.v + N, g.v + 2 * N, g.m, g.f_ext, g.f_ext + N, g.f_ext + 2 * N};
     {
@@ -909,11 +1048,20 @@ __device__ __forceinline__ void mpm_seq_body(const SeqArgs& A, int vb, int vg, i
       const int share = words <= 1 ? NW : (words == 2 ? NW / 2 : 1);  // warps that share a word's runs
       const int word = wid / share, mine = wid % share;
       float* const tile = stg + (copies ? wid % copies : 0) * stride;
-      if (wid < copies) {
+      bool shared_tiles = copies == 1 || copies == 2;
+      if (shared_tiles) {
+        int runs = 0;
+#pragma unroll
+        for (int w = 0; w < NW; ++w) runs += __popc(s_start[w]);
+        shared_tiles = 5 * runs > 2 * ch.y;
+      }
+      if (shared_tiles) {
+        scatter_shared_tiles<REACT>(sp, ch.y, copies, stg, stride, nv, e0, e01, g);
+      } else if (wid < copies) {
         for (int i = lane; i < stride / 4; i += 32) reinterpret_cast<float4*>(tile)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
         __syncwarp();
       }
-      const int rounds = copies ? NW / copies : 1;
+      const int rounds = shared_tiles ? 0 : (copies ? NW / copies : 1);
       for (int round = 0; round < rounds; ++round) {
         if (round > 0) __syncthreads();
         if (copies && wid / copies != round) continue;
