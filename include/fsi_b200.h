@@ -476,7 +476,8 @@ int fsi_mpm_substep(const FsiParticles* pt, const FsiGrid* g, const FsiMpmParams
 /* count, start and chunk must be 16-byte aligned */
 typedef struct FsiMpmBins {
   int32_t n_bins;       /* ceil(n_grid / FSI_BIN_EDGE)^3 */
-  int32_t max_chunks;   /* capacity of chunk[] and of each third of box[] */
+  int32_t max_chunks;   /* capacity of chunk[] and of each third of box[]: fsi_mpm_bins_layout's, or more, which
+                           lets a launch cut few chunks into parts (a record each) */
   int32_t* key;         /* [n_particles] scratch (bin keys, then the in-bin sort) */
   int32_t* count;       /* [n_bins] zero before the first fsi_mpm_bin; kept zero after each call */
   int32_t* start;       /* [n_bins] end offset of each bin in perm after fsi_mpm_bin */
