@@ -269,3 +269,9 @@ def stream_handle(stream=None):
 
     s = stream if stream is not None else torch.cuda.current_stream()
     return ctypes.c_void_p(s.cuda_stream)
+
+
+def overridden(obj, originals):
+    """Whether an object's class or instance replaces one of the methods (name -> function): a fused call that stands
+    for them must then leave them their turn."""
+    return any(name in vars(obj) or getattr(type(obj), name) is not fn for name, fn in originals.items())

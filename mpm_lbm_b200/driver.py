@@ -393,22 +393,31 @@ class FSIDriver3D:
         self._project()
         self.lbm.clear_moving_boundary_force_accumulator()
         S = self.config.lbm_substeps_per_fsi_step
-        t0 = time.perf_counter()
-        self.lbm.update_dynamic_solid(self.config.dynamic_solid_threshold)
-        self.lbm.reinitialize_new_fluid_cells()
-        self._t("coupling_time", t0)
-        t0 = time.perf_counter()
-        # the per-direction reductions are read only after the last substep: the others go to the library in one call
-        # (a substep issued from here costs 12 us of host time, more than a small lattice's substep takes).  phi is
-        # unchanged within the FSI step: the reference's repeated mask updates only copy solid -> old_solid
-        self.lbm.step_moving_bounceback_run(S - 1)
-        if S > 1:
-            self.lbm.mark_repeat_mask_update()
-        self.lbm.dirstats_enabled = True
-        self.lbm.step_moving_bounceback()
-        self.lbm.accumulate_moving_boundary_force_sample()
+        # substeps ahead of the last one that go to the library in one call (a substep issued from here costs 12 us of
+        # host time, more than a small lattice's substep takes); none where a method of a substep is replaced
+        together = 0 if self.lbm.substeps_replaced() else S - 1
+        s = 0
+        while s < S:
+            t0 = time.perf_counter()
+            if s == 0:
+                self.lbm.update_dynamic_solid(self.config.dynamic_solid_threshold)
+            else:
+                # phi is unchanged within the FSI step: the reference's repeat call only copies solid -> old_solid
+                self.lbm.mark_repeat_mask_update()
+            self.lbm.reinitialize_new_fluid_cells()
+            self._t("coupling_time", t0)
+            t0 = time.perf_counter()
+            if s == 0 and together:
+                self.lbm.step_moving_bounceback_run(together)
+                s = together
+            else:
+                # the per-direction reductions are read only after the last substep
+                self.lbm.dirstats_enabled = s == S - 1
+                self.lbm.step_moving_bounceback()
+                self.lbm.accumulate_moving_boundary_force_sample()
+                s += 1
+            self._t("lbm_step_time", t0)
         self.total_lbm_substeps += S
-        self._t("lbm_step_time", t0)
         self.lbm.finalize_moving_boundary_force_accumulator()
         self._advance_mpm_with_moving_boundary_reaction()
 

@@ -21,7 +21,8 @@ import torch
 
 from . import _lib
 from ._lib import (FSI_CELL_OVERRIDE, FSI_CELL_SOLID, FSI_MODE_DIRSTATS, FSI_MODE_MOVING_BB, FSI_MODE_PENALTY,
-                   FSI_MODE_SUBCYCLED, FSI_TUNE_LBM_OCC3, FSI_TUNE_LBM_OCC3_PF, FSI_TUNE_LBM_OCC4, FsiLbmDiag, FsiLbmParams, FsiLbmState, FsiStepCtl, call, ptr, stream_handle)
+                   FSI_MODE_SUBCYCLED, FSI_TUNE_LBM_OCC3, FSI_TUNE_LBM_OCC3_PF, FSI_TUNE_LBM_OCC4, FsiLbmDiag,
+                   FsiLbmParams, FsiLbmState, FsiStepCtl, call, overridden, ptr, stream_handle)
 from .config import (KERNEL_OPEN_BOUNDARY_CODES, LEGACY_EXTERNAL_SOLVER_RELAXATION_PARAMETER,
                      STANDARD_LATTICE_KINEMATIC_VISCOSITY, LBMConfig, tau_from_lattice_kinematic_viscosity,
                      tau_from_legacy_external_solver_parameter)
@@ -431,11 +432,24 @@ class LBMFluid3D:
         self._fused_accumulation = bool(mode & FSI_MODE_SUBCYCLED)
         self._substep(mode)
 
+    def substeps_replaced(self):
+        """Whether a subclass or wrapper replaces a method that belongs to a moving-boundary substep."""
+        return overridden(self, _SUBSTEP)
+
     def step_moving_bounceback_run(self, n):
         """n step_moving_bounceback() without per-direction reductions, each
         followed by accumulate_moving_boundary_force_sample() when the subcycle
-        accumulator is open, through one call of the library (fsi_lbm_substeps)."""
+        accumulator is open, through one call of the library (fsi_lbm_substeps),
+        or one by one where one of these methods is replaced."""
         if n <= 0:
+            return
+        if self.substeps_replaced():
+            dirstats, self.dirstats_enabled = self.dirstats_enabled, False
+            for _ in range(n):
+                self.step_moving_bounceback()
+                if self._accumulating:
+                    self.accumulate_moving_boundary_force_sample()
+            self.dirstats_enabled = dirstats
             return
         if self.tau_f is None:
             raise RuntimeError("init_simulation() must run before stepping")
@@ -740,3 +754,8 @@ class LBMFluid3D:
         np.savez_compressed(f"{out_prefix}_{n}.npz", rho=self.rho.to_numpy(), velocity=self.v.to_numpy(),
                             solid=self.solid.to_numpy(), solid_phi=self.solid_phi.to_numpy(),
                             hydro_force=self.hydro_force.to_numpy(), cell_force=self.cell_force.to_numpy())
+
+
+_SUBSTEP = {name: getattr(LBMFluid3D, name) for name in
+            ("step_moving_bounceback", "accumulate_moving_boundary_force_sample", "mark_repeat_mask_update",
+             "reinitialize_new_fluid_cells")}

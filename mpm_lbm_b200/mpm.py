@@ -15,7 +15,7 @@ import numpy as np
 import torch
 
 from ._lib import (FSI_BIN_CHUNK, FsiCouplingStats, FsiGrid, FsiMpmBins, FsiMpmParams, FsiParticles, call,
-                   ptr, stream_handle)
+                   overridden, ptr, stream_handle)
 from .config import MPMConfig
 from .fields import ParticleField
 
@@ -235,6 +235,14 @@ class MPMSolid3D:
              self._stream())
 
     def substep(self):
+        """clear_grid, p2g, grid_update and g2p (solid.py:212-315) in one call of the library, or one by one where one of
+        them is replaced (by a subclass, on the instance or on the class)."""
+        if overridden(self, _PHASES):
+            self.clear_grid()
+            self.p2g()
+            self.grid_update()
+            self.g2p()
+            return
         self._one_phase_grid()
         call("fsi_mpm_substep", ctypes.byref(self.particles), ctypes.byref(self.grid), ctypes.byref(self.params),
              self._stream())
@@ -393,3 +401,6 @@ class MPMSolid3D:
         np.save(os.path.join(out_dir, f"{prefix}_v.npy"), self.v.to_numpy())
         np.save(os.path.join(out_dir, f"{prefix}_F.npy"), self.F.to_numpy())
         np.save(os.path.join(out_dir, f"{prefix}_J.npy"), self.Jp.to_numpy())
+
+
+_PHASES = {name: getattr(MPMSolid3D, name) for name in ("clear_grid", "p2g", "grid_update", "g2p")}
