@@ -20,6 +20,7 @@
 #include <climits>
 
 #include "common.cuh"
+#include "grid_node.cuh"
 #include "mpm_common.cuh"
 
 namespace fsi {
@@ -277,17 +278,6 @@ __device__ __forceinline__ float bspline_w(float f, int o) {
   return o == 0 ? 0.5f * (1.5f - f) * (1.5f - f) : (o == 1 ? 0.75f - (f - 1.0f) * (f - 1.0f) : 0.5f * (f - 0.5f) * (f - 0.5f));
 }
 
-// One velocity component of a grid node of mass 1 / im after the grid update
-// and the sticky walls (solid.py:97-111, 251-259): momentum and dt times the
-// external force over the mass
-__device__ __forceinline__ float grid_node_component(float P, float im, float f, float gravity, int idx, int G,
-                                                     const FsiMpmParams& mp) {
-  float u = (P + mp.dt * f) * im + mp.dt * gravity;
-  if (idx < mp.bound && u < 0.0f) u = 0.0f;
-  if (idx > G - mp.bound && u > 0.0f) u = 0.0f;
-  return u;
-}
-
 // G2P sums of a particle whose stencil leaves the grid, or whose chunk's node
 // box does not fit the shared-memory stage (bins gone stale): a rolled loop
 // over the nodes inside the grid, from the stage when stg is non-null, from
@@ -316,9 +306,9 @@ __device__ __noinline__ void g2p_slow(const float* stg, int nv, const Box& bx, c
 #pragma unroll
       for (int a = 0; a < 3; ++a) gv[a] = g.v[a * N + node];
       if (m > 0.f) {
-        const float im = __frcp_rn(m);
+        const NodeMass nm = node_mass(m);
 #pragma unroll
-        for (int a = 0; a < 3; ++a) gv[a] = grid_node_component(gv[a], im, f[a], mp.gravity[a], id[a], G, mp);
+        for (int a = 0; a < 3; ++a) gv[a] = grid_node_component(gv[a], nm, f[a], mp.gravity[a], id[a], G, mp);
       }
     }
 #pragma unroll
@@ -839,10 +829,10 @@ __device__ __forceinline__ void mpm_seq_body(const SeqArgs& A, int vb, int vg, i
           const float f[3] = {g.f_ext[node], g.f_ext[N + node], g.f_ext[2 * N + node]};
           float u[3] = {P[0], P[1], P[2]};
           if (m > 0.0f) {
-            const float im = __frcp_rn(m);
-            u[0] = grid_node_component(P[0], im, f[0], mp.gravity[0], I, G, mp);
-            u[1] = grid_node_component(P[1], im, f[1], mp.gravity[1], Jj, G, mp);
-            u[2] = grid_node_component(P[2], im, f[2], mp.gravity[2], K, G, mp);
+            const NodeMass nm = node_mass(m);
+            u[0] = grid_node_component(P[0], nm, f[0], mp.gravity[0], I, G, mp);
+            u[1] = grid_node_component(P[1], nm, f[1], mp.gravity[1], Jj, G, mp);
+            u[2] = grid_node_component(P[2], nm, f[2], mp.gravity[2], K, G, mp);
           }
 #pragma unroll
           for (int a = 0; a < 3; ++a) stg[a * nv + li] = u[a];
