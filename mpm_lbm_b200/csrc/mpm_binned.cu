@@ -715,8 +715,9 @@ __device__ __forceinline__ void mpm_seq_body(const SeqArgs& A, int vb, int vg, i
   const int n = pt.n;
   const int s = A.s;
   const bool do_g2p = s > 0, do_p2g = s < A.M;
-  // the records of the last three substeps are the ones that remain: earlier ones would be overwritten
-  const bool do_stats = REACT && do_p2g && s + 3 >= A.M;
+  // only the record of the last substep remains: each launch zeroes the slot of the substep after its own, so that the
+  // last two zero those of the two substeps before the last
+  const bool do_stats = REACT && s + 1 == A.M;
   const int bg = (s + 2) % 3, bs = s % 3, bz = (s + 1) % 3;
   const int G = A.grid[0].n;
   const int64_t N = (int64_t)G * G * G;
