@@ -644,9 +644,9 @@ __device__ __forceinline__ void accum_max_warp(const Case& c, float nrm) {
 // moving-wall correction and momentum-exchange link force when MOVING
 // (fluid.py:431-440, 488-519).
 template <bool ODD, bool H, bool MOVING>
-__device__ __forceinline__ void store_near_solid(const Case& c, int pp, const Nbh& n, int cell, uint32_t nb, float rho,
+__device__ __forceinline__ void store_near_solid(const Case& c, const Nbh& n, int cell, uint32_t nb, float rho,
                                               const float* out) {
-  float* hpp = c.s.hpp + (int64_t)pp * 3 * c.s.pitch;
+  float* hpp = c.s.hpp + (int64_t)c.c.pp * 3 * c.s.pitch;
   const int64_t P = c.s.pitch;
 #pragma unroll
   for (int s = 0; s < 19; ++s) {
@@ -778,8 +778,7 @@ __device__ __forceinline__ void step_cell_load(const Case& c, int x, int jr, int
 // per-direction link statistics (the caller synchronises the CTA and flushes
 // them).
 template <bool ODD, bool H, bool MOVING, bool BCW, bool PEN>
-__device__ __forceinline__ void step_cell_finish(const Case& c, const FsiStepCtl& ctl, int bx, StepCell& q,
-                                                 DirAcc& acc) {
+__device__ __forceinline__ void step_cell_finish(const Case& c, int bx, StepCell& q, DirAcc& acc) {
   const int lane = threadIdx.x;
   const int nx = c.s.nx, ny = c.s.ny, nz = c.s.nz;
   const int x = q.x;
@@ -788,7 +787,7 @@ __device__ __forceinline__ void step_cell_finish(const Case& c, const FsiStepCtl
   const int j = inrow ? q.jr : 0, k = q.k;
   const int row = k * ny + j;
   const int cell = row * nx + x;
-  const bool dirstats = MOVING && (ctl.mode & FSI_MODE_DIRSTATS);
+  const bool dirstats = MOVING && (c.c.mode & FSI_MODE_DIRSTATS);
   const uint8_t fl = q.fl;
   const bool fluid = !(fl & kSolid);
   const uint32_t nb = q.nb;
@@ -797,7 +796,7 @@ __device__ __forceinline__ void step_cell_finish(const Case& c, const FsiStepCtl
   float* const F = q.F;
 
   // ---- pending open boundary of the previous step (fluid.py:538-569)
-  if (BCW && ctl.bc_pending && inrow) {
+  if (BCW && c.c.bc_pending && inrow) {
     if (c.p.bc_left != 0 && bx == 0) bc_face_warp<0>(c, lane, row, fl, F);
     if (c.p.bc_right != 0 && bx == ((nx - 1) >> 5)) bc_face_warp<1>(c, lane, row, fl, F);
   }
@@ -920,12 +919,12 @@ __device__ __forceinline__ void step_cell_finish(const Case& c, const FsiStepCtl
       }
     } else {
       if (!ODD) make_nbh(c, x, j, k, n);
-      store_near_solid<ODD, H, MOVING>(c, ctl.pp, n, cell, nb, rho, F);
+      store_near_solid<ODD, H, MOVING>(c, n, cell, nb, rho, F);
     }
   } else if (MOVING && valid && (fl & kLink)) {
     // solid cell receiving link forces: recycle last step's ping-pong slot
-    float* prev = c.s.hpp + (int64_t)(ctl.pp ^ 1) * 3 * P;
-    if (ctl.mode & FSI_MODE_SUBCYCLED) {
+    float* prev = c.s.hpp + (int64_t)(c.c.pp ^ 1) * 3 * P;
+    if (c.c.mode & FSI_MODE_SUBCYCLED) {
       float a[3];
 #pragma unroll
       for (int d = 0; d < 3; ++d) {
@@ -982,13 +981,12 @@ __device__ __forceinline__ void dirstats_end(const Case& c, DirAcc& acc, int nth
 // the batched kernel (c staged in shared memory); acc: the CTA's shared
 // per-direction accumulator.
 template <bool ODD, bool H, bool MOVING, bool BCW, bool PEN>
-__device__ __forceinline__ void lbm_step_tile(const Case& c, const FsiStepCtl& ctl, int bx, int by, int bz,
-                                              DirAcc& acc) {
-  const bool dirstats = MOVING && (ctl.mode & FSI_MODE_DIRSTATS);
+__device__ __forceinline__ void lbm_step_tile(const Case& c, int bx, int by, int bz, DirAcc& acc) {
+  const bool dirstats = MOVING && (c.c.mode & FSI_MODE_DIRSTATS);
   if (dirstats) dirstats_begin(acc, 256);
   StepCell q;
   step_cell_load<ODD, H>(c, bx * 32 + (int)threadIdx.x, by * 8 + (int)threadIdx.y, bz, q);
-  step_cell_finish<ODD, H, MOVING, BCW, PEN>(c, ctl, bx, q, acc);
+  step_cell_finish<ODD, H, MOVING, BCW, PEN>(c, bx, q, acc);
   if (dirstats) dirstats_end(c, acc, 256);
 }
 
@@ -1025,7 +1023,7 @@ __global__ void __launch_bounds__(256, MINB) k_lbm_step(const Case c) {
       prefetch_tile_l2<H>(c, (int)(t - r * gx), (int)(r % gy), (int)(r / gy));
     }
   }
-  lbm_step_tile<ODD, H, MOVING, BCW, PEN>(c, c.c, blockIdx.x, blockIdx.y, blockIdx.z, acc);
+  lbm_step_tile<ODD, H, MOVING, BCW, PEN>(c, blockIdx.x, blockIdx.y, blockIdx.z, acc);
 }
 
 // ------------------------------------------- paired step (2 cells/thread) ----
@@ -3042,14 +3040,14 @@ __global__ void __launch_bounds__(256, 3) k_batch_lbm_step(const FsiBatchCase* _
     const int r = t / gx, bx = t - r * gx, by = r % gy, bz = r / gy;
     if (moving) {
       if (odd)
-        lbm_step_tile<true, H, true, false, false>(sc, sc.c, bx, by, bz, acc);
+        lbm_step_tile<true, H, true, false, false>(sc, bx, by, bz, acc);
       else
-        lbm_step_tile<false, H, true, false, false>(sc, sc.c, bx, by, bz, acc);
+        lbm_step_tile<false, H, true, false, false>(sc, bx, by, bz, acc);
     } else {
       if (odd)
-        lbm_step_tile<true, H, false, false, true>(sc, sc.c, bx, by, bz, acc);
+        lbm_step_tile<true, H, false, false, true>(sc, bx, by, bz, acc);
       else
-        lbm_step_tile<false, H, false, false, true>(sc, sc.c, bx, by, bz, acc);
+        lbm_step_tile<false, H, false, false, true>(sc, bx, by, bz, acc);
     }
     __syncthreads();  // acc is reused by the next tile
   }
