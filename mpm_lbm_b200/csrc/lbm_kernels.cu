@@ -57,12 +57,12 @@ __device__ __forceinline__ int64_t pop_index(const Case&, int s, int64_t cell) {
   return (int64_t)(i + (i >> 5) * 576u) + 32 * s;
 }
 
+// Populations are read with plain loads: the step writes them in place, and starts
+// while the launch before still does, so they are not the constant data of the
+// kernel that the read-only path asks for (the two take the same time).
 template <>
 struct Pop<false> {
   static __device__ __forceinline__ float ld(const Case& c, int s, int64_t cell) {
-    return __ldg(static_cast<const float*>(c.s.pop) + pop_index(c, s, cell));
-  }
-  static __device__ __forceinline__ float ld_rw(const Case& c, int s, int64_t cell) {
     return static_cast<const float*>(c.s.pop)[pop_index(c, s, cell)];
   }
   static __device__ __forceinline__ void st(const Case& c, int s, int64_t cell, float v) {
@@ -70,7 +70,7 @@ struct Pop<false> {
   }
   // by block-layout index b (pop_index without the 32 s term)
   static __device__ __forceinline__ float ldb(const Case& c, int s, int64_t b) {
-    return __ldg(static_cast<const float*>(c.s.pop) + b + 32 * s);
+    return static_cast<const float*>(c.s.pop)[b + 32 * s];
   }
   static __device__ __forceinline__ void stb(const Case& c, int s, int64_t b, float v) {
     static_cast<float*>(c.s.pop)[b + 32 * s] = v;
@@ -84,7 +84,6 @@ struct Pop<true> {
     const __half h = static_cast<const __half*>(c.s.pop)[pop_index(c, s, cell)];
     return lattice_w(s) * (c.p.rho0 + __half2float(h));
   }
-  static __device__ __forceinline__ float ld_rw(const Case& c, int s, int64_t cell) { return ld(c, s, cell); }
   static __device__ __forceinline__ void st(const Case& c, int s, int64_t cell, float v) {
     const float inv_w = s == 0 ? 3.0f : (s <= 6 ? 18.0f : 36.0f);
     static_cast<__half*>(c.s.pop)[pop_index(c, s, cell)] = __float2half_rn(__fmaf_rn(v, inv_w, -c.p.rho0));
@@ -139,7 +138,7 @@ __device__ __forceinline__ float decode_pop(const Case& c, const Coord& q, int s
   int ss;
   int64_t sc;
   pop_slot(c, q, cell, fl, nb, s, ss, sc);
-  return Pop<H>::ld_rw(c, ss, sc);
+  return Pop<H>::ld(c, ss, sc);
 }
 
 // ------------------------------------------------------- open boundary ----
@@ -1041,14 +1040,14 @@ struct Pop2;
 template <>
 struct Pop2<false> {
   static __device__ __forceinline__ float2 ld(const Case& c, int s, int64_t cell) {
-    return __ldg(reinterpret_cast<const float2*>(static_cast<const float*>(c.s.pop) + pop_index(c, s, cell)));
+    return *reinterpret_cast<const float2*>(static_cast<const float*>(c.s.pop) + pop_index(c, s, cell));
   }
   static __device__ __forceinline__ void st(const Case& c, int s, int64_t cell, float2 v) {
     *reinterpret_cast<float2*>(static_cast<float*>(c.s.pop) + pop_index(c, s, cell)) = v;
   }
   // by block-layout index b of the pair's first cell (b even)
   static __device__ __forceinline__ float2 ldb(const Case& c, int s, int64_t b) {
-    return __ldg(reinterpret_cast<const float2*>(static_cast<const float*>(c.s.pop) + b + 32 * s));
+    return *reinterpret_cast<const float2*>(static_cast<const float*>(c.s.pop) + b + 32 * s);
   }
   static __device__ __forceinline__ void stb(const Case& c, int s, int64_t b, float2 v) {
     *reinterpret_cast<float2*>(static_cast<float*>(c.s.pop) + b + 32 * s) = v;
@@ -1674,8 +1673,8 @@ __global__ void k_to_natural(const Case c) {
   for (int s = 1; s < 19; s += 2) {
     const int64_t z = nb_cell(c, q, kEx(s), kEy(s), kEz(s));
     if (c.s.flags[z] & kSolid) continue;
-    const float a = Pop<H>::ld_rw(c, s, z);
-    const float b = Pop<H>::ld_rw(c, kOpp(s), i);
+    const float a = Pop<H>::ld(c, s, z);
+    const float b = Pop<H>::ld(c, kOpp(s), i);
     Pop<H>::st(c, s, z, b);
     Pop<H>::st(c, kOpp(s), i, a);
   }
@@ -1792,8 +1791,8 @@ __device__ __forceinline__ void relink_cells(const Case& c, int widx0, int wstri
           const bool old_ff = !c.s.old_solid[y] && !c.s.old_solid[zz];
           const bool new_ff = yf && zf;
           if (old_ff != new_ff) {
-            const float a = Pop<H>::ld_rw(c, sd, zz);
-            const float b = Pop<H>::ld_rw(c, kOpp(sd), y);
+            const float a = Pop<H>::ld(c, sd, zz);
+            const float b = Pop<H>::ld(c, kOpp(sd), y);
             Pop<H>::st(c, sd, zz, b);
             Pop<H>::st(c, kOpp(sd), y, a);
           }
@@ -1901,7 +1900,7 @@ __global__ void k_flush_bc(const Case c) {
 #pragma unroll
       for (int s = 0; s < 19; ++s) {
         pop_slot(c, q, cell, fl, nb, s, ss[s], sc[s]);
-        F[s] = Pop<H>::ld_rw(c, ss[s], sc[s]);
+        F[s] = Pop<H>::ld(c, ss[s], sc[s]);
       }
       apply_face_bc(c.p, c.s.vel_left_dyn, side, in, F, cnt, c.s.diag, c.s.diag, ob_filter_slot(c.s, j, k));
 #pragma unroll

@@ -428,8 +428,7 @@ __device__ __forceinline__ int small_div(int a, float inv) { return (int)(((floa
 // zeroes the first nq of the seven values (momentum, mass, external force) of
 // the nodes of the recorded boxes: warp w of the nw warps that share the work
 // takes the records w, w + nw, ...
-__device__ __forceinline__ void zero_boxes(const FsiGrid& go, const int32_t* __restrict__ rec, int nrec, int w, int nw,
-                                           int nq) {
+__device__ __forceinline__ void zero_boxes(const FsiGrid& go, const int32_t* rec, int nrec, int w, int nw, int nq) {
   const int G = go.n;
   const int64_t N = (int64_t)G * G * G;
   for (int r = w; r < nrec; r += nw) {
