@@ -126,10 +126,14 @@ class MPMSolid3D:
         self._binned_clean = True  # the buffers are zero outside the recorded boxes
         self._binned_mode = "seq"
         self._since_bin = 0
-        # binned substeps between automatic re-binnings.  As particles cross cells a chunk's node box grows (to three
-        # times its nodes within some ten substeps of a moving body) and its scatter with it.  Four substeps, moving /
-        # at rest, every 64 -> every 8: 222,000 particles 403 -> 360 / 287 -> 305 us, 500,000 841 -> 726 / 617 -> 602,
-        # 1,000,000 1,827 -> 1,529 / 1,098 -> 1,080; 98,000 209 -> 216 / 150 -> 186.
+        # binned substeps after which the next call of substeps_binned re-bins first (a call's own substeps run on one
+        # binning).  As particles cross cells a chunk's node box grows, and its staging, tiles and flush with it.  us per
+        # substep in calls of four, every 64 -> every 8, moving by 0.004 to 0.015 cells per substep / at rest:
+        #   1,000,000 particles, 2 per cell  561-618 -> 437-479 / 441 -> 406;  16 per cell  405-461 -> 348-384 / 314 -> 314
+        #     400,000            2 per cell  201-213 -> 174-182 / 167 -> 161;  16 per cell  154-168 -> 139-150 / 120 -> 127
+        #     200,000            2 per cell    89-93 -> 82-86   /  75 -> 77;   16 per cell    74-79 -> 75-80   /  60 -> 69
+        # In one call of 40 substeps re-binning every 8 is no gain: 1,000,000 particles at 8 per cell 299-320 -> 299-308
+        # moving, 250 -> 286 at rest; 400,000 129-139 -> 127-132, 107 -> 121.
         self.rebin_interval = 8 if self.n_particles >= 3 << 17 else 64
 
     def _stream(self):
@@ -347,7 +351,8 @@ class MPMSolid3D:
     def substeps_binned(self, count, coupler=None, lbm=None):
         """`count` substeps through fsi_mpm_substeps_binned (one launch per
         substep: the gather of one substep, the stress, reaction and scatter
-        of the next), re-binning first when the bins are due."""
+        of the next), re-binning first when rebin_interval substeps have run
+        since the last binning."""
         if count <= 0:
             return
         self._ensure_binned()
