@@ -53,12 +53,14 @@ L2_BYTES = 126e6
 
 
 def default_tune(cells: int, nx: int, fp16: bool, open_faces: bool) -> int:
-    """Launch variant of the step kernel where nobody has timed them.  us per step, 3 CTAs / 4 CTAs / 3 CTAs with the
-    L2 prefetch: populations beyond the L2 cache and rows that start a 32-cell block, so that a prefetched line is one
-    warp's: 57.7 / 59.1 / 55.0 (128^3), 144.2 / 146.9 / 132.7 (192x176x160), FP16 149.7 / 143.0 / 139.9; without
-    such rows the prefetch costs more than it gives, 89.8 / 86.5 / 91.7 (150x130x140, open faces).  Below, the fourth
-    CTA pays where a cell takes more instructions, FP16 storage (24.7 / 24.2, 96^3) or open faces (55.0 / 53.1,
-    192x96x96), unless the lattice is a wave or less of CTAs (64x40x40: 7.1 / 7.6); else 20.0 / 20.3 (96^3)."""
+    """Launch variant of the step kernel where nobody has timed them.  us per step of a walled channel, 20 steps of a
+    replayed graph (issued one by one, as by step(), each takes 4-8 us more at the large sizes, and a pass over other
+    inputs a little more again), 3 CTAs / 4 CTAs / 3 CTAs with the L2 prefetch: populations beyond the L2 cache and rows
+    that start a 32-cell block, so that a prefetched line is one warp's: 56.0 / 57.0 / 52.1 (128^3), 139.4 / 140.3 /
+    126.4 (192x176x160), FP16 137.6 / 129.7 / 125.8; without such rows open faces take no prefetch, 89.7 / 86.5 / 91.6
+    (150x130x140).  Below, the fourth CTA pays where a cell takes more instructions, FP16 storage (22.0 / 21.3 / 22.8,
+    96^3) or open faces (18.7 / 18.0 / 19.7, FP16 150x70x51), unless the lattice is a wave or less of CTAs (FP16
+    64x40x40: 5.5 / 6.0 / 5.9); else 17.9 / 18.0 / 19.2 (96^3)."""
     if 19 * cells * (2 if fp16 else 4) > L2_BYTES and nx % 32 == 0:
         return FSI_TUNE_LBM_OCC3_PF
     if (fp16 or open_faces) and cells > 200_000:
