@@ -56,8 +56,10 @@ inline unsigned batch_grid(int64_t units, int n_cases, int resident, int most) {
 // still running; it must call griddep_wait() before touching memory that
 // kernel writes (the wait returns once that grid has completed and its writes
 // are visible; in a kernel launched normally it returns at once).
-// griddep_launch() lets the next such kernel be scheduled; every CTA calls it
-// after its own wait, so the chain never runs more than one grid ahead.
+// griddep_launch() lets the next such kernel be scheduled once every CTA has
+// called it or left; a CTA calls it after its own wait, or leaves before the wait
+// having written nothing.  Some CTA of every launch waits, so that the chain
+// never runs more than one grid ahead.
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

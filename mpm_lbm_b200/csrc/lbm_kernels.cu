@@ -1974,10 +1974,11 @@ __device__ __forceinline__ uint8_t readout_cell(const Case& c, int64_t i, float 
   return fl;
 }
 
-// Reads and writes every population once, at 95 % of the copy bandwidth for
-// 192 x 176 x 160 cells (145 us; 238 us with 64-bit divisions for the cell's
-// coordinates, a neighbour address worked out per population and 88 registers
-// for every cell; 256 x 128 x 128 with a pending boundary 268 -> 146 us).
+// Reads and writes every population once, at 96 % of the copy bandwidth for
+// 192 x 176 x 160 cells (952 MB in 151 us alone, 155 us between events with its
+// call; 238 us with 64-bit divisions for the cell's coordinates, a neighbour
+// address worked out per population and 88 registers for every cell;
+// 256 x 128 x 128 with a pending boundary 268 -> 146 us).
 // Without a pending boundary the face code is left out: 40 registers, not 80.
 template <bool H, bool BC>
 __global__ void __launch_bounds__(128) k_readout(const Case c, float* out_pop, float* out_rho, float* out_vel) {

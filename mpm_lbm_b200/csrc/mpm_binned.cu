@@ -8,7 +8,7 @@
 // their last reader.
 //
 // The per-particle and per-node arithmetic is the one of the one-phase
-// kernels (mpm_common.cuh): solid.py:212-315 and the reaction transfers of
+// kernels (mpm_common.cuh) to rounding: solid.py:212-315 and the reaction transfers of
 // penalty.py:90-129, moving_boundary.py:58-110, link_area.py:84-193.  The
 // order of the sums differs (stencils axis by axis, per-warp tiles, then one
 // global atomic per chunk and touched node value), and a node's velocity is
@@ -361,8 +361,9 @@ enum { kQmass = 36, kQkey = 40, kQn = 44 };
 //
 // What bounds it: where a chunk has an SM to itself, the chain of a warp's
 // dependent instructions (some 2,500 a substep at 5 cycles each) and of the
-// trips to L2; where the SMs hold several, instruction issue.  The bytes (the
-// state of 24,576 particles and the touched nodes) move in 1 us.  So the
+// trips to L2; where the SMs hold four, the same chains four to a scheduler, with
+// a third to half of the issue slots used.  The bytes (the state of 24,576
+// particles and the touched nodes) move in 1 us.  So the
 // arithmetic is arranged for few instructions: no thread repeats another's
 // work, the tensor-product stencils are summed axis by axis (a node costs two
 // multiply-adds per value in the gather), the scatter adds three prepared
@@ -372,9 +373,9 @@ enum { kQmass = 36, kQkey = 40, kQn = 44 };
 // substep overwrites are not formed, and what does not depend on the previous
 // launch is read before its end.
 // One substep, before (two threads per particle, 8 warps, tile with
-// shared-memory atomics) and now, with the binning's share: 19.7 -> 14.9 us
-// (4,096 particles), 24.4 -> 21.7 us (24,576), 124 -> 87 us (196,608); the
-// 16-case batch's 11 launches 1,312 -> 630 us.  Three threads per particle (12
+// shared-memory atomics) and now: 19.7 -> 12.4 us from launch to launch (4,096
+// particles), 23.7 -> 19.5 us (24,576 in the benchmarked duct), 126 -> 82 us
+// (196,608 there); the 16-case batch's 11 launches 1,312 -> 630 us.  Three threads per particle (12
 // warps, one axis each) took 13-21 us at the small sizes but 116 us at 196,608
 // particles and no less than before in a batch.
 // Particles at random positions, with the reaction, at 8 / 2 / 0.5 / 0.125 per
@@ -394,8 +395,8 @@ constexpr int kSeqOcc = 4;          // resident CTAs per SM (by registers and by
 // reaction (512 without), two 585 (1,024), one 1,170 (all that are staged).  A
 // compact chunk of 128 particles at 8 per cell has 120-220 nodes, at 2 per cell
 // 270-440, at one per two cells 440-770.  The size is what four CTAs of an SM
-// can have; a sixth less (243, 486 and 973 nodes) was up to 6 % slower at 0.5 to
-// 4 particles per cell and no faster anywhere.
+// can have; a sixth less (243, 486 and 973 nodes) was 2-6 % slower at 2 to 4
+// particles per cell and 2-3 % faster at 0.5 per cell with the SMs full.
 constexpr int kStageFloats = 8192;
 static_assert(kStageFloats >= 4 * kTileCap && kStageFloats % 4 == 0, "stage holds the lattice box");
 constexpr size_t kSeqSmem = sizeof(float) * (kStageFloats + kQn * kChunk);

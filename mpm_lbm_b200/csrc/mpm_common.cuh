@@ -1,7 +1,9 @@
 // Per-particle and per-node pieces of the MPM substep and of the reaction
 // transfer, shared by the one-phase-per-launch kernels (mpm_kernels.cu) and
-// the binned, shared-memory-staged substep (mpm_binned.cu) so that both paths
-// perform the same arithmetic.
+// the binned, shared-memory-staged substep (mpm_binned.cu).  The two paths share
+// the stress, the reaction force and the state update; the binned one sums the
+// stencils axis by axis and takes a node's velocity from one reciprocal
+// (grid_node.cuh), so that they agree to rounding.
 //
 // Reference semantics:
 //   B-spline weights     src/mpm_lbm/sim/mpm/solid.py:222-230
