@@ -275,7 +275,6 @@ class MPMSolid3D:
         grids[2] = FsiGrid(n=self.n_grid, v=ptr(self.t_gv2), m=ptr(self.t_gm2), f_ext=ptr(self.t_gf2))
         bins = FsiMpmBins(n_bins=nb.value, max_chunks=mc.value, **{k: ptr(v) for k, v in t.items()})
         self._bins = {"t": t, "grids": grids, "struct": bins}
-        self._binned_clean = True
         self._since_bin = None
 
     def _buffers(self, b):
