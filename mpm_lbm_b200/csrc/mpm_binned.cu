@@ -428,16 +428,21 @@ __device__ __forceinline__ int small_div(int a, float inv) { return (int)(((floa
 
 // zeroes the first nq of the seven values (momentum, mass, external force) of
 // the nodes of the recorded boxes: warp w of the nw warps that share the work
-// takes the records w, w + nw, ...
+// takes the records w, w + nw, ...; where there are several warps per record
+// they share it, 32 nodes in turn (SHARE; in the batched kernel, whose arguments
+// are in shared memory, not in constants, the registers for it cost 2 %)
+template <bool SHARE = true>
 __device__ __forceinline__ void zero_boxes(const FsiGrid& go, const int32_t* rec, int nrec, int w, int nw, int nq) {
   const int G = go.n;
   const int64_t N = (int64_t)G * G * G;
-  for (int r = w; r < nrec; r += nw) {
+  const int parts = SHARE ? max(1, nw / max(nrec, 1)) : 1;
+  for (int u = w; u < nrec * parts; u += nw) {
+    const int r = u / parts;
     const Box bx = load_box(rec + 6 * r);
     const int e0 = bx.ext[0], e01 = e0 * bx.ext[1];
     const bool small = bx.vol < (1 << 20);  // the range of small_div
     const float i0 = small_inv(max(e0, 1)), i01 = small_inv(max(e01, 1));
-    for (int li = threadIdx.x & 31; li < bx.vol; li += 32) {
+    for (int li = 32 * (u - r * parts) + (threadIdx.x & 31); li < bx.vol; li += 32 * parts) {
       const int k = small ? small_div(li, i01) : li / e01, q = li - k * e01;
       const int j = small ? small_div(q, i0) : q / e0, i = q - j * e0;
       const int64_t node = ((int64_t)(k + bx.lo[2]) * G + (j + bx.lo[1])) * G + (i + bx.lo[0]);
@@ -696,7 +701,7 @@ __device__ __forceinline__ ReactStats reaction_stats(const ReactParticle& rp, co
 // serialization: what is read before the wait (the chunk table, perm, mass,
 // vol0, fixed) was complete before the launch before the last one, and every
 // launch of the sequence waits for the one before it.
-template <bool REACT>
+template <bool REACT, bool BATCH>
 __device__ __forceinline__ void mpm_seq_body(const SeqArgs& A, int vb, int vg, int max_split) {
   constexpr int T = kSeqT, NW = T / 32;
   constexpr int NQ = REACT ? 7 : 4;  // grid values a substep writes
@@ -775,7 +780,7 @@ __device__ __forceinline__ void mpm_seq_body(const SeqArgs& A, int vb, int vg, i
   const int zero_first = by_idle ? nch : 0;
   if (vb >= nch) {
     if (s >= 2)
-      zero_boxes(grid_of(A, bz), A.box + bz * A.box_stride, A.meta[kMetaRec + bz], (vb - zero_first) * NW + wid,
+      zero_boxes<!BATCH>(grid_of(A, bz), A.box + bz * A.box_stride, A.meta[kMetaRec + bz], (vb - zero_first) * NW + wid,
                  (vg - zero_first) * NW, NQ);
     return;
   }
@@ -1131,7 +1136,7 @@ __device__ __forceinline__ void mpm_seq_body(const SeqArgs& A, int vb, int vg, i
     }
   }
   if (!by_idle && s >= 2)
-    zero_boxes(grid_of(A, bz), A.box + bz * A.box_stride, A.meta[kMetaRec + bz], vb * NW + wid, vg * NW, NQ);
+    zero_boxes<!BATCH>(grid_of(A, bz), A.box + bz * A.box_stride, A.meta[kMetaRec + bz], vb * NW + wid, vg * NW, NQ);
   if (do_stats) {
     // the CTA's part: one global atomic per CTA and quantity
     __syncthreads();
@@ -1169,7 +1174,7 @@ __global__ __launch_bounds__(kSeqT, kSeqOcc) void k_mpm_seq(const __grid_constan
   const int* const w = reinterpret_cast<const int*>(&A);
 #pragma unroll
   for (int i = 0; i < (int)(sizeof(SeqArgs) / 4); i += 16) asm volatile("" ::"r"(w[i]));
-  mpm_seq_body<REACT>(A, blockIdx.x, gridDim.x, 4);
+  mpm_seq_body<REACT, false>(A, blockIdx.x, gridDim.x, 4);
 }
 
 __global__ void k_grid_velocity(FsiGrid g, FsiMpmParams mp, float* __restrict__ out) {
@@ -1444,7 +1449,7 @@ __global__ __launch_bounds__(kSeqT, kSeqOcc) void k_batch_mpm_seq(const FsiBatch
   }
   load_batch_seq(bc, s, M, &A);
   __syncthreads();
-  mpm_seq_body<true>(A, blockIdx.x, gridDim.x, max_split);
+  mpm_seq_body<true, true>(A, blockIdx.x, gridDim.x, max_split);
 }
 
 __global__ __launch_bounds__(kSortT) void k_batch_bin_sort(const FsiBatchCase* __restrict__ cases) {
