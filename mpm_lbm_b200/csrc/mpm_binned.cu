@@ -281,42 +281,57 @@ __device__ __forceinline__ float bspline_w(float f, int o) {
 // G2P sums of a particle whose stencil leaves the grid, or whose chunk's node
 // box does not fit the shared-memory stage (bins gone stale): a rolled loop
 // over the nodes inside the grid, from the stage when stg is non-null, from
-// the grid otherwise, a node's seven values requested together.
+// the grid otherwise.  Three nodes' loads together instead of one's: clouds whose
+// boxes have outgrown the stage (24,576 particles, bins 30 substeps old at 0.3
+// cells a substep) 54 -> 41 us per substep; in the batched kernel the registers
+// for it cost every substep 2 %.
+// U: nodes whose loads are in flight together
+template <int U>
 __device__ __noinline__ void g2p_slow(const float* stg, int nv, const Box& bx, const FsiGrid& g, const FsiMpmParams& mp,
                                       const BSpline& b, float s4, float v[3], float nC[9]) {
   const int G = g.n;
   const int64_t N = (int64_t)G * G * G;
   float sv[3] = {0.f, 0.f, 0.f}, sC[9] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll 1
-  for (int o = 0; o < 27; ++o) {
-    const int ox = o / 9, oy = (o / 3) % 3, oz = o % 3;
-    const int id[3] = {b.base[0] + ox, b.base[1] + oy, b.base[2] + oz};
-    if (id[0] < 0 || id[0] >= G || id[1] < 0 || id[1] >= G || id[2] < 0 || id[2] >= G) continue;
-    const float w = bspline_w(b.fx[0], ox) * bspline_w(b.fx[1], oy) * bspline_w(b.fx[2], oz);
-    const float d[3] = {((float)ox - b.fx[0]) * mp.dx, ((float)oy - b.fx[1]) * mp.dx, ((float)oz - b.fx[2]) * mp.dx};
-    const int li = ((id[2] - bx.lo[2]) * bx.ext[1] + (id[1] - bx.lo[1])) * bx.ext[0] + (id[0] - bx.lo[0]);
-    const int64_t node = ((int64_t)id[2] * G + id[1]) * G + id[0];
-    float gv[3];
-    if (stg) {
+  for (int o0 = 0; o0 < 27; o0 += U) {
+    float P[U][3], f[U][3], m[U];
 #pragma unroll
-      for (int a = 0; a < 3; ++a) gv[a] = stg[a * nv + li];
-    } else {
-      const float m = g.m[node];
-      const float f[3] = {g.f_ext[node], g.f_ext[N + node], g.f_ext[2 * N + node]};  // all in flight together
-#pragma unroll
-      for (int a = 0; a < 3; ++a) gv[a] = g.v[a * N + node];
-      if (m > 0.f) {
-        const NodeMass nm = node_mass(m);
-#pragma unroll
-        for (int a = 0; a < 3; ++a) gv[a] = grid_node_component(gv[a], nm, f[a], mp.gravity[a], id[a], G, mp);
-      }
+    for (int h = 0; h < U; ++h) {
+      const int o = min(o0 + h, 26);
+      const int I = clampi(b.base[0] + o / 9, 0, G - 1), J = clampi(b.base[1] + (o / 3) % 3, 0, G - 1),
+                K = clampi(b.base[2] + o % 3, 0, G - 1);  // a node outside is left out below
+      const int li = ((K - bx.lo[2]) * bx.ext[1] + (J - bx.lo[1])) * bx.ext[0] + (I - bx.lo[0]);
+      const int64_t node = ((int64_t)K * G + J) * G + I;
+      const float* const p = stg ? stg + li : g.v + node;
+      const int64_t step = stg ? nv : N;
+      P[h][0] = p[0];
+      P[h][1] = p[step];
+      P[h][2] = p[2 * step];
+      m[h] = g.m[node];
+      f[h][0] = g.f_ext[node];
+      f[h][1] = g.f_ext[N + node];
+      f[h][2] = g.f_ext[2 * N + node];
     }
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      const float wg = w * gv[a];
-      sv[a] += wg;
+    for (int h = 0; h < U; ++h) {
+      const int o = o0 + h, ox = o / 9, oy = (o / 3) % 3, oz = o % 3;
+      const int id[3] = {b.base[0] + ox, b.base[1] + oy, b.base[2] + oz};
+      if (o >= 27 || id[0] < 0 || id[0] >= G || id[1] < 0 || id[1] >= G || id[2] < 0 || id[2] >= G) continue;
+      const float w = bspline_w(b.fx[0], ox) * bspline_w(b.fx[1], oy) * bspline_w(b.fx[2], oz);
+      const float d[3] = {((float)ox - b.fx[0]) * mp.dx, ((float)oy - b.fx[1]) * mp.dx,
+                          ((float)oz - b.fx[2]) * mp.dx};
+      if (!stg && m[h] > 0.f) {
+        const NodeMass nm = node_mass(m[h]);
 #pragma unroll
-      for (int k = 0; k < 3; ++k) sC[a * 3 + k] += wg * d[k] * s4;
+        for (int a = 0; a < 3; ++a) P[h][a] = grid_node_component(P[h][a], nm, f[h][a], mp.gravity[a], id[a], G, mp);
+      }
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        const float wg = w * P[h][a];
+        sv[a] += wg;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) sC[a * 3 + k] += wg * d[k] * s4;
+      }
     }
   }
 #pragma unroll
@@ -885,7 +900,7 @@ __device__ __forceinline__ void mpm_seq_body(const SeqArgs& A, int vb, int vg, i
             nC[a * 3 + 2] = cz * s4;
           }
         } else {
-          g2p_slow(nv > 0 ? stg : nullptr, nv, bx, g, mp, b, s4, v, nC);
+          g2p_slow<BATCH ? 1 : 3>(nv > 0 ? stg : nullptr, nv, bx, g, mp, b, s4, v, nC);
         }
         float Fo[9];
 #pragma unroll
