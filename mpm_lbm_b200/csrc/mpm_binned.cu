@@ -406,15 +406,25 @@ constexpr int kSeqOcc = 4;          // resident CTAs per SM (by registers and by
 // one region for the staged node velocities (G2P, 3 per node), the reaction's
 // lattice box (4 per cell) and the scatter tiles (7 values per node and copy
 // with the reaction, 4 without): each is written after the last read of the one
-// before it.  Four copies of the tile fit boxes of up to 292 nodes with the
-// reaction (512 without), two 585 (1,024), one 1,170 (all that are staged).  A
-// compact chunk of 128 particles at 8 per cell has 120-220 nodes, at 2 per cell
-// 270-440, at one per two cells 440-770.  The size is what four CTAs of an SM
-// can have; a sixth less (243, 486 and 973 nodes) was 2-6 % slower at 2 to 4
-// particles per cell and 2-3 % faster at 0.5 per cell with the SMs full.
-constexpr int kStageFloats = 8192;
+// before it.  A compact chunk of 128 particles at 8 per cell has boxes of 120-220
+// nodes, at 2 per cell 270-440, at one per two cells 440-770.
+// Where four CTAs of an SM are resident: as large as leaves 60 KB of the SM's
+// memory to the L1 cache, whose lines hold the loads in flight (the particle
+// state, scattered when the particles are in random order).  Four tiles fit 234
+// nodes with the reaction (410 without), two 468 (820), one 937 (all that are
+// staged).  8,192 floats (292, 585 and 1,170 nodes), which leave 28 KB, took
+// 775 us, not 633, per substep of 10^6 particles in random order, 248, not 225 us,
+// in order; 105, not 87, and 70.5, not 67.5 us for 196,608 (the latter with the
+// reaction); only at one particle per cell, 100, not 106 us.
+constexpr int kStageFloats = 6560;
+// Two CTAs per SM, for clouds of less than 48 full chunks with the reaction and
+// for few box records: four tiles for 438 nodes with the reaction (768 without),
+// two for 877, one for all.  4,096 particles at 8 per cell, with the reaction, on
+// 32^3 and 80^3 nodes: 13.5 -> 12.1 and 12.7 -> 11.8 us per substep; a step of ten
+// substeps of a plate in a 75 x 52 x 61 box (two of them) 425 -> 403 us.
+constexpr int kWideStageFloats = 12288;
 static_assert(kStageFloats >= 4 * kTileCap && kStageFloats % 4 == 0, "stage holds the lattice box");
-constexpr size_t kSeqSmem = sizeof(float) * (kStageFloats + kQn * kChunk);
+constexpr size_t seq_smem(int stage) { return sizeof(float) * (stage + kQn * kChunk); }
 
 struct SeqArgs {
   FsiParticles pt;
@@ -712,17 +722,17 @@ __device__ __forceinline__ ReactStats reaction_stats(const ReactParticle& rp, co
 }
 
 // launch A.s of the sequence for the chunks vb, vb + vg, ... (kSeqT threads,
-// kSeqSmem bytes of dynamic shared memory), launched with programmatic stream
+// seq_smem(STAGE) bytes of dynamic shared memory), launched with programmatic stream
 // serialization: what is read before the wait (the chunk table, perm, mass,
 // vol0, fixed) was complete before the launch before the last one, and every
 // launch of the sequence waits for the one before it.
-template <bool REACT, bool BATCH>
+template <bool REACT, bool BATCH, int STAGE>
 __device__ __forceinline__ void mpm_seq_body(const SeqArgs& A, int vb, int vg, int max_split) {
   constexpr int T = kSeqT, NW = T / 32;
   constexpr int NQ = REACT ? 7 : 4;  // grid values a substep writes
   extern __shared__ float4 seq_smem4[];
   float* const stg = reinterpret_cast<float*>(seq_smem4);  // node velocities, then the lattice box, then the tiles
-  float* const sp = stg + kStageFloats;                    // [kChunk][kQn] P2G payload
+  float* const sp = stg + STAGE;                           // [kChunk][kQn] P2G payload
   __shared__ int s_lo[3], s_hi[3];
   __shared__ unsigned s_start[NW];  // bit i of word w: particle 32 w + i starts a run of one base node
   __shared__ float s_scale;
@@ -939,7 +949,7 @@ __device__ __forceinline__ void mpm_seq_body(const SeqArgs& A, int vb, int vg, i
     const bool staged = bx.vol <= kTileCap;
     const int nv = staged ? bx.vol : 0;
     const int stride = (NQ * nv + 3) & ~3;  // floats of a tile
-    const int copies = !staged ? 0 : (4 * stride <= kStageFloats ? 4 : (2 * stride <= kStageFloats ? 2 : (stride <= kStageFloats)));
+    const int copies = !staged ? 0 : (4 * stride <= STAGE ? 4 : (2 * stride <= STAGE ? 2 : (stride <= STAGE)));
     if (tid == 0) {
       int32_t* const out = A.box + bs * A.box_stride + 6 * c;
 #pragma unroll
@@ -1182,14 +1192,14 @@ __global__ __launch_bounds__(kSeqT) void k_mpm_seq_prologue(const __grid_constan
   seq_prologue_body(A, blockIdx.x, gridDim.x);
 }
 
-template <bool REACT>
+template <bool REACT, int STAGE>
 __global__ __launch_bounds__(kSeqT, kSeqOcc) void k_mpm_seq(const __grid_constant__ SeqArgs A) {
   // the launch's arguments into the constant caches while the previous launch
   // still runs (a first access after the wait costs a trip to L2)
   const int* const w = reinterpret_cast<const int*>(&A);
 #pragma unroll
   for (int i = 0; i < (int)(sizeof(SeqArgs) / 4); i += 16) asm volatile("" ::"r"(w[i]));
-  mpm_seq_body<REACT, false>(A, blockIdx.x, gridDim.x, 4);
+  mpm_seq_body<REACT, false, STAGE>(A, blockIdx.x, gridDim.x, 4);
 }
 
 __global__ void k_grid_velocity(FsiGrid g, FsiMpmParams mp, float* __restrict__ out) {
@@ -1252,8 +1262,15 @@ int sm_count() { return device_sm_count(); }
 
 inline unsigned nblk(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
 
-// CTAs of a fused-sequence launch: one resident wave (at most one CTA per chunk)
-int seq_ctas(bool react, int max_chunks, int* ctas) {
+using SeqKernel = void (*)(const SeqArgs);
+
+SeqKernel seq_kernel(bool react, bool wide) {
+  return react ? (wide ? k_mpm_seq<true, kWideStageFloats> : k_mpm_seq<true, kStageFloats>)
+               : (wide ? k_mpm_seq<false, kWideStageFloats> : k_mpm_seq<false, kStageFloats>);
+}
+
+// CTAs of a fused-sequence launch, one resident wave (at most one CTA per chunk), and whether their stage is the wide one
+int seq_ctas(bool react, int n, int max_chunks, int* ctas, bool* wide) {
   static int occ[64][2] = {};
   int dev = 0;
   int rc = cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
@@ -1261,16 +1278,21 @@ int seq_ctas(bool react, int max_chunks, int* ctas) {
   if (dev < 0 || dev >= 64) return invalid("device ordinal out of range");
   int& o = occ[dev][react ? 1 : 0];
   if (!o) {
-    void (*k)(const SeqArgs) = react ? k_mpm_seq<true> : k_mpm_seq<false>;
-    if ((rc = cuda_check(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSeqSmem),
-                         "k_mpm_seq shared memory")))
-      return rc;
+    for (const bool w : {false, true})
+      if ((rc = cuda_check(cudaFuncSetAttribute(seq_kernel(react, w), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                (int)seq_smem(w ? kWideStageFloats : kStageFloats)),
+                           "k_mpm_seq shared memory")))
+        return rc;
     int b = 0;
-    if ((rc = cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k, kSeqT, kSeqSmem), "k_mpm_seq occupancy")))
+    if ((rc = cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, seq_kernel(react, false), kSeqT,
+                                                                       seq_smem(kStageFloats)),
+                         "k_mpm_seq occupancy")))
       return rc;
     o = b > 0 ? b : 1;
   }
-  *ctas = std::max(1, std::min(max_chunks, sm_count() * o));
+  // (without the reaction's three values a small cloud's tiles fit, and its chunks are cut further with four CTAs)
+  *wide = max_chunks <= 2 * sm_count() || (react && n < 48 * kChunk);
+  *ctas = std::max(1, std::min(max_chunks, sm_count() * (*wide ? 2 : o)));
   return FSI_OK;
 }
 
@@ -1357,14 +1379,15 @@ extern "C" int fsi_mpm_substeps_binned(const FsiParticles* pt, const FsiGrid gri
   }
   A.M = n_substeps;
   int ctas = 0;
-  if ((rc = seq_ctas(cp != nullptr, bins->max_chunks, &ctas))) return rc;
+  bool wide = false;
+  if ((rc = seq_ctas(cp != nullptr, pt->n, bins->max_chunks, &ctas, &wide))) return rc;
+  const size_t smem = seq_smem(wide ? kWideStageFloats : kStageFloats);
   cudaStream_t st = (cudaStream_t)stream;
   cudaError_t lerr = launch_pdl(k_mpm_seq_prologue, dim3(ctas), dim3(kSeqT), 0, st, A);
   if ((rc = cuda_check(lerr, "k_mpm_seq_prologue (launch)")) || (rc = launch_check("k_mpm_seq_prologue"))) return rc;
   for (int i = 0; i <= n_substeps; ++i) {
     A.s = i;
-    lerr = cp ? launch_pdl(k_mpm_seq<true>, dim3(ctas), dim3(kSeqT), kSeqSmem, st, A)
-              : launch_pdl(k_mpm_seq<false>, dim3(ctas), dim3(kSeqT), kSeqSmem, st, A);
+    lerr = launch_pdl(seq_kernel(cp != nullptr, wide), dim3(ctas), dim3(kSeqT), smem, st, A);
     if ((rc = cuda_check(lerr, "k_mpm_seq (launch)")) || (rc = launch_check("k_mpm_seq"))) return rc;
   }
   return FSI_OK;
@@ -1464,7 +1487,7 @@ __global__ __launch_bounds__(kSeqT, kSeqOcc) void k_batch_mpm_seq(const FsiBatch
   }
   load_batch_seq(bc, s, M, &A);
   __syncthreads();
-  mpm_seq_body<true, true>(A, blockIdx.x, gridDim.x, max_split);
+  mpm_seq_body<true, true, kStageFloats>(A, blockIdx.x, gridDim.x, max_split);
 }
 
 __global__ __launch_bounds__(kSortT) void k_batch_bin_sort(const FsiBatchCase* __restrict__ cases) {
@@ -1514,7 +1537,7 @@ extern "C" int fsi_batch_mpm_substeps(FsiBatchCase* cases, const FsiBatchDims* d
     if (dev < 0 || dev >= 64) return invalid("device ordinal out of range");
     if (!attr_set[dev]) {
       if ((rc = cuda_check(cudaFuncSetAttribute(k_batch_mpm_seq, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                (int)kSeqSmem),
+                                                (int)seq_smem(kStageFloats)),
                            "k_batch_mpm_seq shared memory")))
         return rc;
       attr_set[dev] = true;
@@ -1532,8 +1555,8 @@ extern "C" int fsi_batch_mpm_substeps(FsiBatchCase* cases, const FsiBatchDims* d
   const int64_t chunks = (int64_t)nblk(d->max_particles, kChunk) * d->n_cases, room = (int64_t)sm_count() * kSeqOcc;
   const int max_split = chunks * 4 <= room ? 4 : (chunks * 2 <= room ? 2 : 1);
   for (int i = 0; i <= n_substeps; ++i) {
-    const cudaError_t lerr = launch_pdl(k_batch_mpm_seq, gc, dim3(kSeqT), kSeqSmem, st, (const FsiBatchCase*)cases, i,
-                                        n_substeps, max_split);
+    const cudaError_t lerr = launch_pdl(k_batch_mpm_seq, gc, dim3(kSeqT), seq_smem(kStageFloats), st,
+                                        (const FsiBatchCase*)cases, i, n_substeps, max_split);
     if ((rc = cuda_check(lerr, "k_batch_mpm_seq (launch)")) || (rc = launch_check("k_batch_mpm_seq"))) return rc;
   }
   return FSI_OK;

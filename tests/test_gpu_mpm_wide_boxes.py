@@ -1,10 +1,13 @@
 """Chunks whose node box leaves room for one or two scatter tiles, whose warps then
 divide the grid values between them or take turns: boxes on both sides of every
-limit (with the reaction 292, 585 and 1,170 nodes, without 512 and 1,024), from
-three particles a chunk up, runs of one base node on both sides of 2.5
-particles, many particles in one cell of a wide box, chunks cut into parts, stencils
-that leave the grid, and bins gone stale.  Compared with the CPU oracle like the
-other chunk shapes, under the same tolerances."""
+limit (four, two and one tile: with the reaction 438, 877 and 1,331 nodes, without
+768 and 1,331; with many box records, where the tiles have less room and chunks are
+cut into parts, 234, 468 and 937, without 410 and 820), from three particles a chunk
+up, runs of one base node on both sides of 2.5 particles, many particles in one cell
+of a wide box, stencils that leave the grid, and bins gone stale.  Compared with the
+CPU oracle like the other chunk shapes, under the same tolerances."""
+
+import sys
 
 import numpy as np
 import pytest
@@ -17,7 +20,7 @@ BINS = np.stack(np.meshgrid(*[np.arange(4)] * 3, indexing="ij"), -1).reshape(-1,
 
 
 def _bins_of(ext, per_bin, rng, run=1):
-    """All 64 bins (too many to be cut into parts) with per_bin particles each, `run` of them in a cell, whose stencils
+    """All 64 bins (with few box records too many to be cut into parts) with per_bin particles each, `run` of them in a cell, whose stencils
     span ext nodes per axis."""
     lo, hi = 0.01, np.array(ext) - 2 - 0.03
     x = rng.uniform(0.0, 1.0, (64, -(-per_bin // run), 3)) * (hi - lo) + lo
@@ -31,32 +34,43 @@ def _cloud(kind, rng):
     if kind == "one_cell_of_a_wide_box":  # 60 particles with one stencil and 35 over the bin
         x = _bins_of((9, 9, 10), 95, rng).reshape(64, 95, 3)
         x[:, 35:] = x[:, 35:36].round() + rng.uniform(0.01, 0.9, (64, 60, 3)) - 0.49
-        return np.clip(x.reshape(-1, 3), 1.0, 31.0), (400, 1000), 95
+        return np.clip(x.reshape(-1, 3), 1.0, 31.0), (27, 1000), 95
     if kind == "parts":  # one chunk, cut into parts of 25 particles
-        return 8.51 + rng.uniform(0, 7.9, (100, 3)), (293, 1000), 100
+        return 8.51 + rng.uniform(0, 7.9, (100, 3)), (100, 1000), 100
     if kind == "leaving_the_grid":  # the bin at the upper corner, clamped at 1 - dx
         return np.minimum(24.51 + rng.uniform(0, 7.5, (90, 3)), 31.0), (100, 900), 90
     ext, per_bin, run = kind
     nodes = int(np.prod(ext))
-    return _bins_of(ext, per_bin, rng, run), (nodes, nodes), per_bin
+    return _bins_of(ext, per_bin, rng, run), (nodes if RECORDS == "few" else 27, nodes), per_bin
 
 
-FRESH = [((5, 7, 8), 64, 1), ((6, 7, 7), 64, 1), ((8, 8, 8), 3, 1), ((6, 9, 10), 31, 2), ((8, 8, 9), 33, 1),
-         ((8, 8, 9), 90, 3), ((6, 10, 10), 94, 2), ((6, 10, 10), 93, 3), ((9, 9, 10), 3, 1), ((9, 10, 10), 95, 2),
+FRESH = [((5, 7, 8), 64, 1), ((6, 8, 9), 64, 1), ((7, 7, 9), 3, 1), ((6, 9, 10), 31, 2), ((8, 8, 9), 33, 1),
+         ((8, 8, 9), 90, 3), ((8, 9, 10), 94, 2), ((8, 10, 10), 93, 3), ((9, 9, 10), 3, 1), ((9, 10, 10), 95, 2),
          ((10, 10, 10), 95, 1), ((10, 10, 10), 95, 3)]
 STALE = [((9, 10, 11), 95, 1), ((10, 10, 11), 60, 2), ((10, 11, 11), 95, 1), ((11, 11, 11), 90, 3), ((11, 11, 12), 64, 1)]
+RECORDS = "few"
+
+
+@pytest.fixture(params=["few", "many"])
+def records(request, monkeypatch):
+    """Box records for the chunks only, or (as large clouds have) for every CTA of the device."""
+    from mpm_lbm_b200 import mpm
+
+    if request.param == "many":
+        monkeypatch.setattr(mpm, "FSI_BIN_CHUNK", 1)
+    monkeypatch.setattr(sys.modules[__name__], "RECORDS", request.param)
+    monkeypatch.setattr(chunks, "_cloud", _cloud)
 
 
 @pytest.mark.parametrize("kind", FRESH + ["one_cell_of_a_wide_box", "parts", "leaving_the_grid"], ids=str)
 @pytest.mark.parametrize("react", [False, True])
-def test_wide_boxes_match_oracle(kind, react, monkeypatch):
-    monkeypatch.setattr(chunks, "_cloud", _cloud)
+def test_wide_boxes_match_oracle(kind, react, records):
     chunks.test_chunk_shapes_match_oracle(kind, react)
 
 
 @pytest.mark.parametrize("kind", STALE, ids=str)
 @pytest.mark.parametrize("react", [False, True])
-def test_stale_bins_match_oracle(kind, react, monkeypatch):
+def test_stale_bins_match_oracle(kind, react, records, monkeypatch):
     import torch
 
     from mpm_lbm_b200.mpm import MPMSolid3D
@@ -71,7 +85,6 @@ def test_stale_bins_match_oracle(kind, react, monkeypatch):
         self.t_x.copy_(x)
 
     monkeypatch.setattr(MPMSolid3D, "rebin", from_the_centres)
-    monkeypatch.setattr(chunks, "_cloud", _cloud)
     chunks.test_chunk_shapes_match_oracle(kind, react)
 
 
