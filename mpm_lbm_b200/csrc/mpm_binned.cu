@@ -388,15 +388,15 @@ enum { kQmass = 36, kQkey = 40, kQn = 44 };
 // substep overwrites are not formed, and what does not depend on the previous
 // launch is read before its end.
 // One substep, before (two threads per particle, 8 warps, tile with
-// shared-memory atomics) and now: 19.7 -> 12.4 us from launch to launch (4,096
-// particles), 23.7 -> 19.5 us (24,576 in the benchmarked duct), 126 -> 82 us
-// (196,608 there); the 16-case batch's 11 launches 1,312 -> 630 us.  Three threads per particle (12
-// warps, one axis each) took 13-21 us at the small sizes but 116 us at 196,608
-// particles and no less than before in a batch.
+// shared-memory atomics) and now: 19.7 -> 12.2 us from launch to launch (4,096
+// particles), 23.7 -> 18.5 us (24,576 in the benchmarked duct), 126 -> 77 us
+// (196,608 there); the 16-case batch's 11 launches 1,312 -> 630-650 us.  Three
+// threads per particle (12 warps, one axis each) took 13-21 us at the small sizes
+// but 116 us at 196,608 particles and no less than before in a batch.
 // Particles at random positions, with the reaction, at 8 / 2 / 0.5 / 0.125 per
 // cell, that earlier form and this one: 24,576 particles 23 / 24 / 28 / 58 us and
-// 18 / 21 / 25 / 36 us; 196,608: 105 / 129 / 183 / 359 us and
-// 70 / 93 / 144 / 218 us.
+// 18 / 21 / 24 / 37 us; 196,608: 105 / 129 / 183 / 359 us and
+// 67 / 92 / 133 / 217 us.
 
 // bins->meta: [0] chunks, [1 + b] records in box[b], [4] chunks scattered
 // without a tile, [5 + b] buffer b holds recorded boxes not yet zeroed

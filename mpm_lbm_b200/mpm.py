@@ -129,11 +129,11 @@ class MPMSolid3D:
         # binned substeps after which the next call of substeps_binned re-bins first (a call's own substeps run on one
         # binning).  As particles cross cells a chunk's node box grows, and its staging, tiles and flush with it.  us per
         # substep in calls of four, every 64 -> every 8, moving by 0.004 to 0.015 cells per substep / at rest:
-        #   1,000,000 particles, 2 per cell  561-618 -> 437-479 / 441 -> 406;  16 per cell  405-461 -> 348-384 / 314 -> 314
-        #     400,000            2 per cell  201-213 -> 174-182 / 167 -> 161;  16 per cell  154-168 -> 139-150 / 120 -> 127
-        #     200,000            2 per cell    89-93 -> 82-86   /  75 -> 77;   16 per cell    74-79 -> 75-80   /  60 -> 69
-        # In one call of 40 substeps re-binning every 8 is no gain: 1,000,000 particles at 8 per cell 299-320 -> 299-308
-        # moving, 250 -> 286 at rest; 400,000 129-139 -> 127-132, 107 -> 121.
+        #   1,000,000 particles, 2 per cell  474-495 -> 393-397 / 419 -> 366;  16 per cell  377-384 -> 312-343 / 280 -> 283
+        #     400,000            2 per cell  187-195 -> 161-165 / 154 -> 146;  16 per cell  141-157 -> 127-137 / 108 -> 115
+        #     200,000            2 per cell    84-88 -> 79-82   /  70 -> 72;   16 per cell    69-73 -> 70-75   /  54 -> 63
+        # In one call of 40 substeps re-binning every 8 is no gain: 1,000,000 particles at 8 per cell 268-289 -> 267-284
+        # moving, 218 -> 249 at rest; 400,000 120-128 -> 118-124, 96 -> 109.
         self.rebin_interval = 8 if self.n_particles >= 3 << 17 else 64
 
     def _stream(self):
