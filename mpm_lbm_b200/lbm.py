@@ -447,11 +447,13 @@ class LBMFluid3D:
             return
         if self.substeps_replaced():
             dirstats, self.dirstats_enabled = self.dirstats_enabled, False
-            for _ in range(n):
-                self.step_moving_bounceback()
-                if self._accumulating:
-                    self.accumulate_moving_boundary_force_sample()
-            self.dirstats_enabled = dirstats
+            try:
+                for _ in range(n):
+                    self.step_moving_bounceback()
+                    if self._accumulating:
+                        self.accumulate_moving_boundary_force_sample()
+            finally:
+                self.dirstats_enabled = dirstats
             return
         if self.tau_f is None:
             raise RuntimeError("init_simulation() must run before stepping")

@@ -91,3 +91,15 @@ def test_replaced_substep_method_is_reached(calls, name, times, substeps):
 def test_own_substeps_go_in_one_call(calls, substeps):
     _subcycled(lbm_module.LBMFluid3D, substeps)
     assert calls.count("fsi_lbm_substeps") == (substeps > 1) and calls.count("fsi_lbm_substep") == 1
+
+
+def test_substeps_that_end_in_an_error_leave_the_statistics_on(calls):
+    class Fluid(lbm_module.LBMFluid3D):
+        def step_moving_bounceback(self):
+            raise ValueError("stop")
+
+    lbm = Fluid(LBMConfig(nx=8, ny=8, nz=8), device="cpu")
+    lbm.tau_f = 0.6
+    with pytest.raises(ValueError, match="stop"):
+        lbm.step_moving_bounceback_run(2)
+    assert lbm.dirstats_enabled
